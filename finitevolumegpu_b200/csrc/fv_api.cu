@@ -7,6 +7,10 @@
 // host loop (GPUSimulators/Simulator.py:176-217) with one launch, and one
 // synchronisation, per 100-step dt interval, where the reference reads back
 // min(cfl_data).
+//
+// The file is compiled once for the runtime and, with FV_PART set to a scheme's
+// number, once per scheme for that scheme's kernels, so that the parts build in
+// parallel.
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -33,8 +37,15 @@
 using fv::SimCtl;
 using fv::StageArgs;
 
+#ifdef FV_PART
+constexpr int kPart = FV_PART;
+#else
+constexpr int kPart = -1;
+#endif
+
 namespace {
 
+#ifndef FV_PART
 thread_local std::string g_err;
 
 int fail(int code, const char* fmt, ...) {
@@ -62,79 +73,94 @@ int fail(int code, const char* fmt, ...) {
 int scheme_nv(int scheme) { return scheme == FV_EE2D_KP07_DIMSPLIT ? 4 : 3; }
 int scheme_ghost(int scheme) { return (scheme == FV_LXF || scheme == FV_FORCE || scheme == FV_HLL) ? 1 : 2; }
 
+#endif  // FV_PART
+
 using KernelFn = void (*)(StageArgs);
+using BatchFn = void (*)(fv::BatchArgs);
+
+// The kernels of a table row, in the part that compiles them.
+template <int S, int... P>
+constexpr KernelFn stage_fn() {
+    if constexpr (S == kPart) return fv::stage_kernel<S, P...>;
+    else return nullptr;
+}
+template <int S, int... P>
+constexpr BatchFn batch_fn() {
+    if constexpr (S == kPart) return fv::batched_stage_kernel<S, P...>;
+    else return nullptr;
+}
 
 struct KEntry {
     int scheme;
     int W, H, NT;
     bool split;
-    KernelFn fn;
+    mutable KernelFn fn;  // set by link_tables
 };
 
 // Tile configurations per scheme; the first entry of a scheme is its default.
 const KEntry kTable[] = {
-    {FV_KP07_DIMSPLIT, 124, 60, 256, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 124, 60, 256>},
-    {FV_KP07_DIMSPLIT, 124, 28, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 124, 28, 128>},
-    {FV_KP07_DIMSPLIT, 60, 28, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 60, 28, 128>},
-    {FV_KP07_DIMSPLIT, 28, 28, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 28, 28, 128>},
-    {FV_HLL2, 124, 60, 256, true, fv::stage_kernel<fv::HLL2, 124, 60, 256>},
-    {FV_HLL2, 124, 28, 128, true, fv::stage_kernel<fv::HLL2, 124, 28, 128>},
-    {FV_HLL2, 28, 28, 128, true, fv::stage_kernel<fv::HLL2, 28, 28, 128>},
-    {FV_HLL2, 60, 28, 128, true, fv::stage_kernel<fv::HLL2, 60, 28, 128>},
-    {FV_WAF, 124, 60, 256, true, fv::stage_kernel<fv::WAF, 124, 60, 256>},
-    {FV_WAF, 124, 28, 128, true, fv::stage_kernel<fv::WAF, 124, 28, 128>},
-    {FV_WAF, 28, 28, 128, true, fv::stage_kernel<fv::WAF, 28, 28, 128>},
-    {FV_WAF, 60, 28, 128, true, fv::stage_kernel<fv::WAF, 60, 28, 128>},
-    {FV_FORCE, 124, 60, 256, true, fv::stage_kernel<fv::FORCE, 124, 60, 256>},
-    {FV_FORCE, 124, 28, 128, true, fv::stage_kernel<fv::FORCE, 124, 28, 128>},
-    {FV_FORCE, 28, 28, 128, true, fv::stage_kernel<fv::FORCE, 28, 28, 128>},
-    {FV_FORCE, 60, 28, 128, true, fv::stage_kernel<fv::FORCE, 60, 28, 128>},
-    {FV_HLL, 124, 60, 256, true, fv::stage_kernel<fv::HLL, 124, 60, 256>},
-    {FV_HLL, 124, 28, 128, true, fv::stage_kernel<fv::HLL, 124, 28, 128>},
-    {FV_HLL, 60, 28, 128, true, fv::stage_kernel<fv::HLL, 60, 28, 128>},
-    {FV_HLL, 28, 28, 128, true, fv::stage_kernel<fv::HLL, 28, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 128, true, fv::stage_kernel<fv::EE2D, 124, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 124, 60, 256, true, fv::stage_kernel<fv::EE2D, 124, 60, 256>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 128, true, fv::stage_kernel<fv::EE2D, 60, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 128, true, fv::stage_kernel<fv::EE2D, 28, 28, 128>},
-    {FV_LXF, 120, 60, 256, false, fv::stage_kernel<fv::LXF, 120, 60, 256>},
-    {FV_LXF, 120, 28, 128, false, fv::stage_kernel<fv::LXF, 120, 28, 128>},
-    {FV_LXF, 120, 60, 128, false, fv::stage_kernel<fv::LXF, 120, 60, 128>},
-    {FV_LXF, 60, 28, 128, false, fv::stage_kernel<fv::LXF, 60, 28, 128>},
-    {FV_KP07, 120, 28, 128, false, fv::stage_kernel<fv::KP07, 120, 28, 128>},
-    {FV_KP07, 120, 60, 128, false, fv::stage_kernel<fv::KP07, 120, 60, 128>},
-    {FV_KP07, 120, 60, 256, false, fv::stage_kernel<fv::KP07, 120, 60, 256>},
-    {FV_KP07, 60, 28, 128, false, fv::stage_kernel<fv::KP07, 60, 28, 128>},
+    {FV_KP07_DIMSPLIT, 124, 60, 256, true, stage_fn<fv::KP07_DIMSPLIT, 124, 60, 256>()},
+    {FV_KP07_DIMSPLIT, 124, 28, 128, true, stage_fn<fv::KP07_DIMSPLIT, 124, 28, 128>()},
+    {FV_KP07_DIMSPLIT, 60, 28, 128, true, stage_fn<fv::KP07_DIMSPLIT, 60, 28, 128>()},
+    {FV_KP07_DIMSPLIT, 28, 28, 128, true, stage_fn<fv::KP07_DIMSPLIT, 28, 28, 128>()},
+    {FV_HLL2, 124, 60, 256, true, stage_fn<fv::HLL2, 124, 60, 256>()},
+    {FV_HLL2, 124, 28, 128, true, stage_fn<fv::HLL2, 124, 28, 128>()},
+    {FV_HLL2, 28, 28, 128, true, stage_fn<fv::HLL2, 28, 28, 128>()},
+    {FV_HLL2, 60, 28, 128, true, stage_fn<fv::HLL2, 60, 28, 128>()},
+    {FV_WAF, 124, 60, 256, true, stage_fn<fv::WAF, 124, 60, 256>()},
+    {FV_WAF, 124, 28, 128, true, stage_fn<fv::WAF, 124, 28, 128>()},
+    {FV_WAF, 28, 28, 128, true, stage_fn<fv::WAF, 28, 28, 128>()},
+    {FV_WAF, 60, 28, 128, true, stage_fn<fv::WAF, 60, 28, 128>()},
+    {FV_FORCE, 124, 60, 256, true, stage_fn<fv::FORCE, 124, 60, 256>()},
+    {FV_FORCE, 124, 28, 128, true, stage_fn<fv::FORCE, 124, 28, 128>()},
+    {FV_FORCE, 28, 28, 128, true, stage_fn<fv::FORCE, 28, 28, 128>()},
+    {FV_FORCE, 60, 28, 128, true, stage_fn<fv::FORCE, 60, 28, 128>()},
+    {FV_HLL, 124, 60, 256, true, stage_fn<fv::HLL, 124, 60, 256>()},
+    {FV_HLL, 124, 28, 128, true, stage_fn<fv::HLL, 124, 28, 128>()},
+    {FV_HLL, 60, 28, 128, true, stage_fn<fv::HLL, 60, 28, 128>()},
+    {FV_HLL, 28, 28, 128, true, stage_fn<fv::HLL, 28, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 128, true, stage_fn<fv::EE2D, 124, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 124, 60, 256, true, stage_fn<fv::EE2D, 124, 60, 256>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 128, true, stage_fn<fv::EE2D, 60, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 128, true, stage_fn<fv::EE2D, 28, 28, 128>()},
+    {FV_LXF, 120, 60, 256, false, stage_fn<fv::LXF, 120, 60, 256>()},
+    {FV_LXF, 120, 28, 128, false, stage_fn<fv::LXF, 120, 28, 128>()},
+    {FV_LXF, 120, 60, 128, false, stage_fn<fv::LXF, 120, 60, 128>()},
+    {FV_LXF, 60, 28, 128, false, stage_fn<fv::LXF, 60, 28, 128>()},
+    {FV_KP07, 120, 28, 128, false, stage_fn<fv::KP07, 120, 28, 128>()},
+    {FV_KP07, 120, 60, 128, false, stage_fn<fv::KP07, 120, 60, 128>()},
+    {FV_KP07, 120, 60, 256, false, stage_fn<fv::KP07, 120, 60, 256>()},
+    {FV_KP07, 60, 28, 128, false, stage_fn<fv::KP07, 60, 28, 128>()},
     // two lines per thread in packed FP32 (same cells, bit for bit)
-    {FV_KP07_DIMSPLIT, 124, 28, 64, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 124, 28, 64, 0, 2>},
-    {FV_KP07_DIMSPLIT, 124, 60, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 124, 60, 128, 0, 2>},
-    {FV_KP07_DIMSPLIT, 60, 28, 64, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 60, 28, 64, 0, 2>},
-    {FV_HLL2, 124, 28, 64, true, fv::stage_kernel<fv::HLL2, 124, 28, 64, 0, 2>},
-    {FV_HLL2, 124, 60, 128, true, fv::stage_kernel<fv::HLL2, 124, 60, 128, 0, 2>},
-    {FV_HLL2, 60, 28, 64, true, fv::stage_kernel<fv::HLL2, 60, 28, 64, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 64, true, fv::stage_kernel<fv::EE2D, 124, 28, 64, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 124, 60, 128, true, fv::stage_kernel<fv::EE2D, 124, 60, 128, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 64, true, fv::stage_kernel<fv::EE2D, 60, 28, 64, 0, 2>},
-    {FV_WAF, 124, 28, 64, true, fv::stage_kernel<fv::WAF, 124, 28, 64, 0, 2>},
-    {FV_WAF, 124, 60, 128, true, fv::stage_kernel<fv::WAF, 124, 60, 128, 0, 2>},
-    {FV_WAF, 60, 28, 64, true, fv::stage_kernel<fv::WAF, 60, 28, 64, 0, 2>},
+    {FV_KP07_DIMSPLIT, 124, 28, 64, true, stage_fn<fv::KP07_DIMSPLIT, 124, 28, 64, 0, 2>()},
+    {FV_KP07_DIMSPLIT, 124, 60, 128, true, stage_fn<fv::KP07_DIMSPLIT, 124, 60, 128, 0, 2>()},
+    {FV_KP07_DIMSPLIT, 60, 28, 64, true, stage_fn<fv::KP07_DIMSPLIT, 60, 28, 64, 0, 2>()},
+    {FV_HLL2, 124, 28, 64, true, stage_fn<fv::HLL2, 124, 28, 64, 0, 2>()},
+    {FV_HLL2, 124, 60, 128, true, stage_fn<fv::HLL2, 124, 60, 128, 0, 2>()},
+    {FV_HLL2, 60, 28, 64, true, stage_fn<fv::HLL2, 60, 28, 64, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 64, true, stage_fn<fv::EE2D, 124, 28, 64, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 124, 60, 128, true, stage_fn<fv::EE2D, 124, 60, 128, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 64, true, stage_fn<fv::EE2D, 60, 28, 64, 0, 2>()},
+    {FV_WAF, 124, 28, 64, true, stage_fn<fv::WAF, 124, 28, 64, 0, 2>()},
+    {FV_WAF, 124, 60, 128, true, stage_fn<fv::WAF, 124, 60, 128, 0, 2>()},
+    {FV_WAF, 60, 28, 64, true, stage_fn<fv::WAF, 60, 28, 64, 0, 2>()},
     // 8-segment rows (120 wide, padded pitch 136): twice the warps of the 124-wide packed tiles
-    {FV_KP07_DIMSPLIT, 120, 28, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 120, 28, 128, 0, 2>},
-    {FV_KP07_DIMSPLIT, 120, 60, 256, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 120, 60, 256, 0, 2>},
-    {FV_HLL2, 120, 28, 128, true, fv::stage_kernel<fv::HLL2, 120, 28, 128, 0, 2>},
-    {FV_HLL2, 120, 60, 256, true, fv::stage_kernel<fv::HLL2, 120, 60, 256, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 120, 28, 128, true, fv::stage_kernel<fv::EE2D, 120, 28, 128, 0, 2>},
-    {FV_WAF, 120, 28, 128, true, fv::stage_kernel<fv::WAF, 120, 28, 128, 0, 2>},
-    {FV_WAF, 120, 60, 256, true, fv::stage_kernel<fv::WAF, 120, 60, 256, 0, 2>},
+    {FV_KP07_DIMSPLIT, 120, 28, 128, true, stage_fn<fv::KP07_DIMSPLIT, 120, 28, 128, 0, 2>()},
+    {FV_KP07_DIMSPLIT, 120, 60, 256, true, stage_fn<fv::KP07_DIMSPLIT, 120, 60, 256, 0, 2>()},
+    {FV_HLL2, 120, 28, 128, true, stage_fn<fv::HLL2, 120, 28, 128, 0, 2>()},
+    {FV_HLL2, 120, 60, 256, true, stage_fn<fv::HLL2, 120, 60, 256, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 120, 28, 128, true, stage_fn<fv::EE2D, 120, 28, 128, 0, 2>()},
+    {FV_WAF, 120, 28, 128, true, stage_fn<fv::WAF, 120, 28, 128, 0, 2>()},
+    {FV_WAF, 120, 60, 256, true, stage_fn<fv::WAF, 120, 60, 256, 0, 2>()},
     // 60 x 60: fewer halo rows per tile than 60 x 28 at the same warps per SM
-    {FV_KP07_DIMSPLIT, 60, 60, 128, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>},
-    {FV_KP07_DIMSPLIT, 60, 60, 256, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 60, 60, 256, 0, 1>},
-    {FV_HLL2, 60, 60, 128, true, fv::stage_kernel<fv::HLL2, 60, 60, 128, 0, 2>},
-    {FV_HLL2, 60, 60, 256, true, fv::stage_kernel<fv::HLL2, 60, 60, 256, 0, 1>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 128, true, fv::stage_kernel<fv::EE2D, 60, 60, 128, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 256, true, fv::stage_kernel<fv::EE2D, 60, 60, 256, 0, 1>},
-    {FV_WAF, 60, 60, 128, true, fv::stage_kernel<fv::WAF, 60, 60, 128, 0, 2>},
-    {FV_WAF, 60, 60, 256, true, fv::stage_kernel<fv::WAF, 60, 60, 256, 0, 1>},
+    {FV_KP07_DIMSPLIT, 60, 60, 128, true, stage_fn<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>()},
+    {FV_KP07_DIMSPLIT, 60, 60, 256, true, stage_fn<fv::KP07_DIMSPLIT, 60, 60, 256, 0, 1>()},
+    {FV_HLL2, 60, 60, 128, true, stage_fn<fv::HLL2, 60, 60, 128, 0, 2>()},
+    {FV_HLL2, 60, 60, 256, true, stage_fn<fv::HLL2, 60, 60, 256, 0, 1>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 128, true, stage_fn<fv::EE2D, 60, 60, 128, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 256, true, stage_fn<fv::EE2D, 60, 60, 256, 0, 1>()},
+    {FV_WAF, 60, 60, 128, true, stage_fn<fv::WAF, 60, 60, 128, 0, 2>()},
+    {FV_WAF, 60, 60, 256, true, stage_fn<fv::WAF, 60, 60, 256, 0, 1>()},
     // Short chains for grids of few tiles, where a substep takes as long as one
     // tile: a walker reconstructs its segment's cells and two more one after the
     // other, 3 + 2 along x and 2 + 2 along y for 12 x 12, 7 + 2 and 4 + 2 for
@@ -144,24 +170,24 @@ const KEntry kTable[] = {
     // 512 x 512 with 28 x 28 by 224 threads 11.3, by 128 13.1.  The halo work of
     // 12 x 12, 1.8 times that of 28 x 28, costs more than it saves from about
     // 512 x 512 on.
-    {FV_KP07_DIMSPLIT, 12, 12, 96, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 12, 12, 96>},
-    {FV_KP07_DIMSPLIT, 28, 28, 224, true, fv::stage_kernel<fv::KP07_DIMSPLIT, 28, 28, 224>},
-    {FV_HLL2, 12, 12, 96, true, fv::stage_kernel<fv::HLL2, 12, 12, 96>},
-    {FV_HLL2, 28, 28, 224, true, fv::stage_kernel<fv::HLL2, 28, 28, 224>},
-    {FV_WAF, 12, 12, 96, true, fv::stage_kernel<fv::WAF, 12, 12, 96>},
-    {FV_WAF, 28, 28, 224, true, fv::stage_kernel<fv::WAF, 28, 28, 224>},
-    {FV_FORCE, 12, 12, 96, true, fv::stage_kernel<fv::FORCE, 12, 12, 96>},
-    {FV_FORCE, 28, 28, 224, true, fv::stage_kernel<fv::FORCE, 28, 28, 224>},
-    {FV_HLL, 12, 12, 96, true, fv::stage_kernel<fv::HLL, 12, 12, 96>},
-    {FV_HLL, 28, 28, 224, true, fv::stage_kernel<fv::HLL, 28, 28, 224>},
-    {FV_EE2D_KP07_DIMSPLIT, 12, 12, 96, true, fv::stage_kernel<fv::EE2D, 12, 12, 96>},
-    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 224, true, fv::stage_kernel<fv::EE2D, 28, 28, 224>},
+    {FV_KP07_DIMSPLIT, 12, 12, 96, true, stage_fn<fv::KP07_DIMSPLIT, 12, 12, 96>()},
+    {FV_KP07_DIMSPLIT, 28, 28, 224, true, stage_fn<fv::KP07_DIMSPLIT, 28, 28, 224>()},
+    {FV_HLL2, 12, 12, 96, true, stage_fn<fv::HLL2, 12, 12, 96>()},
+    {FV_HLL2, 28, 28, 224, true, stage_fn<fv::HLL2, 28, 28, 224>()},
+    {FV_WAF, 12, 12, 96, true, stage_fn<fv::WAF, 12, 12, 96>()},
+    {FV_WAF, 28, 28, 224, true, stage_fn<fv::WAF, 28, 28, 224>()},
+    {FV_FORCE, 12, 12, 96, true, stage_fn<fv::FORCE, 12, 12, 96>()},
+    {FV_FORCE, 28, 28, 224, true, stage_fn<fv::FORCE, 28, 28, 224>()},
+    {FV_HLL, 12, 12, 96, true, stage_fn<fv::HLL, 12, 12, 96>()},
+    {FV_HLL, 28, 28, 224, true, stage_fn<fv::HLL, 28, 28, 224>()},
+    {FV_EE2D_KP07_DIMSPLIT, 12, 12, 96, true, stage_fn<fv::EE2D, 12, 12, 96>()},
+    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 224, true, stage_fn<fv::EE2D, 28, 28, 224>()},
     // the unsplit column walk in row segments of 7 and 4 rows instead of 14:
     // KP07 256 x 256 11.5 and 11.3 us per step instead of 15.4, LxF 4.1 instead of 4.7
-    {FV_LXF, 60, 28, 256, false, fv::stage_kernel<fv::LXF, 60, 28, 256>},
-    {FV_LXF, 60, 28, 448, false, fv::stage_kernel<fv::LXF, 60, 28, 448>},
-    {FV_KP07, 60, 28, 256, false, fv::stage_kernel<fv::KP07, 60, 28, 256>},
-    {FV_KP07, 60, 28, 448, false, fv::stage_kernel<fv::KP07, 60, 28, 448>},
+    {FV_LXF, 60, 28, 256, false, stage_fn<fv::LXF, 60, 28, 256>()},
+    {FV_LXF, 60, 28, 448, false, stage_fn<fv::LXF, 60, 28, 448>()},
+    {FV_KP07, 60, 28, 256, false, stage_fn<fv::KP07, 60, 28, 256>()},
+    {FV_KP07, 60, 28, 448, false, stage_fn<fv::KP07, 60, 28, 448>()},
 };
 constexpr int kNumEntries = sizeof(kTable) / sizeof(kTable[0]);
 
@@ -174,7 +200,7 @@ struct VEntry {
     KEntry k;
 };
 const VEntry kVariantTable[] = {
-#define FV_V(S, ES, V) {V, {S, 124, 60, 256, true, fv::stage_kernel<ES, 124, 60, 256, V>}}
+#define FV_V(S, ES, V) {V, {S, 124, 60, 256, true, stage_fn<ES, 124, 60, 256, V>()}}
     FV_V(FV_HLL, fv::HLL, 1), FV_V(FV_HLL, fv::HLL, 2),
     FV_V(FV_WAF, fv::WAF, 1), FV_V(FV_WAF, fv::WAF, 2), FV_V(FV_WAF, fv::WAF, 3), FV_V(FV_WAF, fv::WAF, 4),
     FV_V(FV_WAF, fv::WAF, 5), FV_V(FV_WAF, fv::WAF, 6), FV_V(FV_WAF, fv::WAF, 7), FV_V(FV_WAF, fv::WAF, 8),
@@ -182,46 +208,45 @@ const VEntry kVariantTable[] = {
 };
 constexpr int kNumVariants = sizeof(kVariantTable) / sizeof(kVariantTable[0]);
 
-using BatchFn = void (*)(fv::BatchArgs);
 struct BEntry {
     int scheme;
     int W, H, NT;
-    BatchFn fn;
+    mutable BatchFn fn;  // set by link_tables
 };
 // Batched kernels; the first entry of a scheme is its default.
 const BEntry kBatchTable[] = {
-    {FV_LXF, 60, 28, 128, fv::batched_stage_kernel<fv::LXF, 60, 28, 128>},
-    {FV_LXF, 120, 28, 128, fv::batched_stage_kernel<fv::LXF, 120, 28, 128>},
-    {FV_KP07, 60, 28, 128, fv::batched_stage_kernel<fv::KP07, 60, 28, 128>},
-    {FV_KP07, 120, 28, 128, fv::batched_stage_kernel<fv::KP07, 120, 28, 128>},
-    {FV_KP07_DIMSPLIT, 60, 28, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 60, 28, 128>},
-    {FV_KP07_DIMSPLIT, 124, 28, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 124, 28, 128>},
-    {FV_KP07_DIMSPLIT, 124, 60, 256, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 124, 60, 256>},
-    {FV_KP07_DIMSPLIT, 28, 28, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 28, 28, 128>},
-    {FV_HLL, 60, 28, 128, fv::batched_stage_kernel<fv::HLL, 60, 28, 128>},
-    {FV_HLL, 124, 28, 128, fv::batched_stage_kernel<fv::HLL, 124, 28, 128>},
-    {FV_HLL, 124, 60, 256, fv::batched_stage_kernel<fv::HLL, 124, 60, 256>},
-    {FV_HLL, 28, 28, 128, fv::batched_stage_kernel<fv::HLL, 28, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 128, fv::batched_stage_kernel<fv::EE2D, 60, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 128, fv::batched_stage_kernel<fv::EE2D, 124, 28, 128>},
-    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 128, fv::batched_stage_kernel<fv::EE2D, 28, 28, 128>},
-    {FV_HLL2, 60, 28, 128, fv::batched_stage_kernel<fv::HLL2, 60, 28, 128>},
-    {FV_HLL2, 124, 28, 128, fv::batched_stage_kernel<fv::HLL2, 124, 28, 128>},
-    {FV_HLL2, 28, 28, 128, fv::batched_stage_kernel<fv::HLL2, 28, 28, 128>},
-    {FV_WAF, 60, 28, 128, fv::batched_stage_kernel<fv::WAF, 60, 28, 128>},
-    {FV_WAF, 124, 28, 128, fv::batched_stage_kernel<fv::WAF, 124, 28, 128>},
-    {FV_WAF, 28, 28, 128, fv::batched_stage_kernel<fv::WAF, 28, 28, 128>},
-    {FV_FORCE, 60, 28, 128, fv::batched_stage_kernel<fv::FORCE, 60, 28, 128>},
-    {FV_FORCE, 124, 28, 128, fv::batched_stage_kernel<fv::FORCE, 124, 28, 128>},
-    {FV_FORCE, 28, 28, 128, fv::batched_stage_kernel<fv::FORCE, 28, 28, 128>},
+    {FV_LXF, 60, 28, 128, batch_fn<fv::LXF, 60, 28, 128>()},
+    {FV_LXF, 120, 28, 128, batch_fn<fv::LXF, 120, 28, 128>()},
+    {FV_KP07, 60, 28, 128, batch_fn<fv::KP07, 60, 28, 128>()},
+    {FV_KP07, 120, 28, 128, batch_fn<fv::KP07, 120, 28, 128>()},
+    {FV_KP07_DIMSPLIT, 60, 28, 128, batch_fn<fv::KP07_DIMSPLIT, 60, 28, 128>()},
+    {FV_KP07_DIMSPLIT, 124, 28, 128, batch_fn<fv::KP07_DIMSPLIT, 124, 28, 128>()},
+    {FV_KP07_DIMSPLIT, 124, 60, 256, batch_fn<fv::KP07_DIMSPLIT, 124, 60, 256>()},
+    {FV_KP07_DIMSPLIT, 28, 28, 128, batch_fn<fv::KP07_DIMSPLIT, 28, 28, 128>()},
+    {FV_HLL, 60, 28, 128, batch_fn<fv::HLL, 60, 28, 128>()},
+    {FV_HLL, 124, 28, 128, batch_fn<fv::HLL, 124, 28, 128>()},
+    {FV_HLL, 124, 60, 256, batch_fn<fv::HLL, 124, 60, 256>()},
+    {FV_HLL, 28, 28, 128, batch_fn<fv::HLL, 28, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 28, 128, batch_fn<fv::EE2D, 60, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 124, 28, 128, batch_fn<fv::EE2D, 124, 28, 128>()},
+    {FV_EE2D_KP07_DIMSPLIT, 28, 28, 128, batch_fn<fv::EE2D, 28, 28, 128>()},
+    {FV_HLL2, 60, 28, 128, batch_fn<fv::HLL2, 60, 28, 128>()},
+    {FV_HLL2, 124, 28, 128, batch_fn<fv::HLL2, 124, 28, 128>()},
+    {FV_HLL2, 28, 28, 128, batch_fn<fv::HLL2, 28, 28, 128>()},
+    {FV_WAF, 60, 28, 128, batch_fn<fv::WAF, 60, 28, 128>()},
+    {FV_WAF, 124, 28, 128, batch_fn<fv::WAF, 124, 28, 128>()},
+    {FV_WAF, 28, 28, 128, batch_fn<fv::WAF, 28, 28, 128>()},
+    {FV_FORCE, 60, 28, 128, batch_fn<fv::FORCE, 60, 28, 128>()},
+    {FV_FORCE, 124, 28, 128, batch_fn<fv::FORCE, 124, 28, 128>()},
+    {FV_FORCE, 28, 28, 128, batch_fn<fv::FORCE, 28, 28, 128>()},
     // 60 x 60, two lines per thread in packed FP32 (same cells, bit for bit)
-    {FV_KP07_DIMSPLIT, 60, 60, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>},
-    {FV_HLL2, 60, 60, 128, fv::batched_stage_kernel<fv::HLL2, 60, 60, 128, 0, 2>},
-    {FV_WAF, 60, 60, 128, fv::batched_stage_kernel<fv::WAF, 60, 60, 128, 0, 2>},
-    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 128, fv::batched_stage_kernel<fv::EE2D, 60, 60, 128, 0, 2>},
+    {FV_KP07_DIMSPLIT, 60, 60, 128, batch_fn<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>()},
+    {FV_HLL2, 60, 60, 128, batch_fn<fv::HLL2, 60, 60, 128, 0, 2>()},
+    {FV_WAF, 60, 60, 128, batch_fn<fv::WAF, 60, 60, 128, 0, 2>()},
+    {FV_EE2D_KP07_DIMSPLIT, 60, 60, 128, batch_fn<fv::EE2D, 60, 60, 128, 0, 2>()},
     // (tile indices that tuner caches may hold)
-    {FV_KP07_DIMSPLIT, 60, 60, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>},
-    {FV_KP07_DIMSPLIT, 124, 28, 128, fv::batched_stage_kernel<fv::KP07_DIMSPLIT, 124, 28, 128>},
+    {FV_KP07_DIMSPLIT, 60, 60, 128, batch_fn<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>()},
+    {FV_KP07_DIMSPLIT, 124, 28, 128, batch_fn<fv::KP07_DIMSPLIT, 124, 28, 128>()},
 };
 constexpr int kNumBatchEntries = sizeof(kBatchTable) / sizeof(kBatchTable[0]);
 
@@ -231,13 +256,61 @@ struct VBEntry {
     BEntry b;
 };
 const VBEntry kBatchVariantTable[] = {
-#define FV_V(S, ES, V) {V, {S, 60, 28, 128, fv::batched_stage_kernel<ES, 60, 28, 128, V>}}
+#define FV_V(S, ES, V) {V, {S, 60, 28, 128, batch_fn<ES, 60, 28, 128, V>()}}
     FV_V(FV_HLL, fv::HLL, 1), FV_V(FV_HLL, fv::HLL, 2),
     FV_V(FV_WAF, fv::WAF, 1), FV_V(FV_WAF, fv::WAF, 2), FV_V(FV_WAF, fv::WAF, 3), FV_V(FV_WAF, fv::WAF, 4),
     FV_V(FV_WAF, fv::WAF, 5), FV_V(FV_WAF, fv::WAF, 6), FV_V(FV_WAF, fv::WAF, 7), FV_V(FV_WAF, fv::WAF, 8),
 #undef FV_V
 };
 constexpr int kNumBatchVariants = sizeof(kBatchVariantTable) / sizeof(kBatchVariantTable[0]);
+
+#ifdef FV_PART
+}  // namespace
+
+// This part's kernels into the tables of the runtime.
+#define FV_CAT2(a, b) a##b
+#define FV_CAT(a, b) FV_CAT2(a, b)
+void FV_CAT(fv_internal_kernels_, FV_PART)(KernelFn* stage, KernelFn* variant, BatchFn* batch, BatchFn* batch_variant) {
+    for (int i = 0; i < kNumEntries; ++i)
+        if (kTable[i].fn) stage[i] = kTable[i].fn;
+    for (int i = 0; i < kNumVariants; ++i)
+        if (kVariantTable[i].k.fn) variant[i] = kVariantTable[i].k.fn;
+    for (int i = 0; i < kNumBatchEntries; ++i)
+        if (kBatchTable[i].fn) batch[i] = kBatchTable[i].fn;
+    for (int i = 0; i < kNumBatchVariants; ++i)
+        if (kBatchVariantTable[i].b.fn) batch_variant[i] = kBatchVariantTable[i].b.fn;
+}
+
+#else
+}  // namespace
+
+#define FV_LINK(K) void fv_internal_kernels_##K(KernelFn*, KernelFn*, BatchFn*, BatchFn*)
+FV_LINK(0);
+FV_LINK(1);
+FV_LINK(2);
+FV_LINK(3);
+FV_LINK(4);
+FV_LINK(5);
+FV_LINK(6);
+FV_LINK(7);
+#undef FV_LINK
+
+namespace {
+
+// The tables' kernels, from the parts, when the library is loaded.
+bool link_tables() {
+    KernelFn stage[kNumEntries] = {}, variant[kNumVariants] = {};
+    BatchFn batch[kNumBatchEntries] = {}, batch_variant[kNumBatchVariants] = {};
+    const auto parts = {fv_internal_kernels_0, fv_internal_kernels_1, fv_internal_kernels_2, fv_internal_kernels_3,
+                        fv_internal_kernels_4, fv_internal_kernels_5, fv_internal_kernels_6, fv_internal_kernels_7};
+    for (const auto part : parts) part(stage, variant, batch, batch_variant);
+    for (int i = 0; i < kNumEntries; ++i) kTable[i].fn = stage[i];
+    for (int i = 0; i < kNumVariants; ++i) kVariantTable[i].k.fn = variant[i];
+    for (int i = 0; i < kNumBatchEntries; ++i) kBatchTable[i].fn = batch[i];
+    for (int i = 0; i < kNumBatchVariants; ++i) kBatchVariantTable[i].b.fn = batch_variant[i];
+    return true;
+}
+const bool g_tables_linked = link_tables();
 
 bool scheme_split(int scheme) { return scheme != FV_LXF && scheme != FV_KP07; }
 
@@ -1865,3 +1938,5 @@ int fv_batch_tile(fv_batch* b, int* tile_w, int* tile_h, int* threads, int* grid
 }
 
 }  // extern "C"
+
+#endif  // FV_PART
