@@ -4,7 +4,7 @@
 // reference, GPUSimulators/Common.py:741-755), a device control block with t,
 // nt, dt and the buffer parity, progress counters of its tiles and one TMA
 // descriptor per buffer and variable.  simulate() reproduces the reference's
-// host loop (GPUSimulators/Simulator.py:176-217) with one launch, and one
+// host loop (GPUSimulators/Simulator.py:176-217) with one run of tasks, and one
 // synchronisation, per 100-step dt interval, where the reference reads back
 // min(cfl_data).
 //
@@ -43,6 +43,14 @@ constexpr int kPart = FV_PART;
 constexpr int kPart = -1;
 #endif
 
+using KernelFn = void (*)(StageArgs);
+using BatchFn = void (*)(fv::BatchArgs);
+// The forms of a stage kernel.
+struct StageFns {
+    KernelFn once = nullptr;  // a CTA per task
+    KernelFn loop = nullptr;  // CTAs that take task after task
+};
+
 namespace {
 
 #ifndef FV_PART
@@ -75,14 +83,11 @@ int scheme_ghost(int scheme) { return (scheme == FV_LXF || scheme == FV_FORCE ||
 
 #endif  // FV_PART
 
-using KernelFn = void (*)(StageArgs);
-using BatchFn = void (*)(fv::BatchArgs);
-
 // The kernels of a table row, in the part that compiles them.
-template <int S, int... P>
-constexpr KernelFn stage_fn() {
-    if constexpr (S == kPart) return fv::stage_kernel<S, P...>;
-    else return nullptr;
+template <int S, int W, int H, int NT, int VAR = 0, int LPT = 1>
+constexpr StageFns stage_fn() {
+    if constexpr (S == kPart) return {fv::stage_kernel<S, W, H, NT, VAR, LPT>, fv::stage_kernel<S, W, H, NT, VAR, LPT, true>};
+    else return {};
 }
 template <int S, int... P>
 constexpr BatchFn batch_fn() {
@@ -94,7 +99,7 @@ struct KEntry {
     int scheme;
     int W, H, NT;
     bool split;
-    mutable KernelFn fn;  // set by link_tables
+    mutable StageFns fn;  // set by link_tables
 };
 
 // Tile configurations per scheme; the first entry of a scheme is its default.
@@ -270,11 +275,11 @@ constexpr int kNumBatchVariants = sizeof(kBatchVariantTable) / sizeof(kBatchVari
 // This part's kernels into the tables of the runtime.
 #define FV_CAT2(a, b) a##b
 #define FV_CAT(a, b) FV_CAT2(a, b)
-void FV_CAT(fv_internal_kernels_, FV_PART)(KernelFn* stage, KernelFn* variant, BatchFn* batch, BatchFn* batch_variant) {
+void FV_CAT(fv_internal_kernels_, FV_PART)(StageFns* stage, StageFns* variant, BatchFn* batch, BatchFn* batch_variant) {
     for (int i = 0; i < kNumEntries; ++i)
-        if (kTable[i].fn) stage[i] = kTable[i].fn;
+        if (kTable[i].fn.once) stage[i] = kTable[i].fn;
     for (int i = 0; i < kNumVariants; ++i)
-        if (kVariantTable[i].k.fn) variant[i] = kVariantTable[i].k.fn;
+        if (kVariantTable[i].k.fn.once) variant[i] = kVariantTable[i].k.fn;
     for (int i = 0; i < kNumBatchEntries; ++i)
         if (kBatchTable[i].fn) batch[i] = kBatchTable[i].fn;
     for (int i = 0; i < kNumBatchVariants; ++i)
@@ -284,7 +289,7 @@ void FV_CAT(fv_internal_kernels_, FV_PART)(KernelFn* stage, KernelFn* variant, B
 #else
 }  // namespace
 
-#define FV_LINK(K) void fv_internal_kernels_##K(KernelFn*, KernelFn*, BatchFn*, BatchFn*)
+#define FV_LINK(K) void fv_internal_kernels_##K(StageFns*, StageFns*, BatchFn*, BatchFn*)
 FV_LINK(0);
 FV_LINK(1);
 FV_LINK(2);
@@ -299,7 +304,7 @@ namespace {
 
 // The tables' kernels, from the parts, when the library is loaded.
 bool link_tables() {
-    KernelFn stage[kNumEntries] = {}, variant[kNumVariants] = {};
+    StageFns stage[kNumEntries] = {}, variant[kNumVariants] = {};
     BatchFn batch[kNumBatchEntries] = {}, batch_variant[kNumBatchVariants] = {};
     const auto parts = {fv_internal_kernels_0, fv_internal_kernels_1, fv_internal_kernels_2, fv_internal_kernels_3,
                         fv_internal_kernels_4, fv_internal_kernels_5, fv_internal_kernels_6, fv_internal_kernels_7};
@@ -587,6 +592,15 @@ struct fv_context {
     char name[256] = {0};
     HostStaging staging;
     CtlSlab ctl_slab;
+    std::atomic<int> running{0};  // simulations in simulate() or advance()
+};
+
+// A simulation's looping kernel with one of its tiles.
+struct LoopForm {
+    const KEntry* ke = nullptr;
+    dim3 grid;              // tiles along x and y
+    unsigned resident = 0;  // CTAs that the GPU holds at once
+    alignas(64) CUtensorMap tmap[2][4];
 };
 
 struct fv_sim {
@@ -611,6 +625,7 @@ struct fv_sim {
     cudaStream_t stream = nullptr;
     alignas(64) StageArgs args;
     size_t smem = 0;         // dynamic shared memory of a launch (stage_smem)
+    LoopForm loop, wide;     // the looping forms (loop_form), once needed
     long long launches = 0;  // stage-kernel launches so far
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
@@ -824,6 +839,37 @@ size_t stage_smem(const fv_context* ctx, size_t tile_bytes, size_t tiles) {
     return std::max(tile_bytes, cap > ctx->smem_reserved ? cap - ctx->smem_reserved : 0);
 }
 
+cudaError_t allow_smem_of(KernelFn fn, size_t bytes) {
+    const void* f = reinterpret_cast<const void*>(fn);
+    const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (r != cudaSuccess) return r;
+    return cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
+// Counts a simulation as one of those that share the GPU, while it runs.
+struct Running {
+    fv_context* ctx;
+    explicit Running(fv_context* c) : ctx(c) { ctx->running.fetch_add(1, std::memory_order_relaxed); }
+    ~Running() { ctx->running.fetch_sub(1, std::memory_order_relaxed); }
+};
+
+// The tensor maps of a simulation's planes with an entry's tile.
+int encode_maps(const fv_sim* s, const KEntry& e, CUtensorMap (*maps)[4]) {
+    const auto enc = encode_fn();
+    for (int b = 0; b < 2; ++b)
+        for (int v = 0; v < s->nv; ++v) {
+            cuuint64_t dims[2] = {(cuuint64_t)(s->nx + 8), (cuuint64_t)(s->ny + 4)};
+            cuuint64_t strides[1] = {(cuuint64_t)s->pitch * sizeof(float)};
+            cuuint32_t box[2] = {(cuuint32_t)entry_box_w(e), (cuuint32_t)(e.H + 4)};
+            cuuint32_t estr[2] = {1, 1};
+            CUresult r = enc(&maps[b][v], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, s->buf[b][v], dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) return fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+        }
+    return FV_OK;
+}
+
 // The part of a launch that differs from call to call.
 struct StagePlan {
     int first_substep = 0, n_sub = 1, steps = 0;
@@ -834,7 +880,69 @@ struct StagePlan {
     int n_tail = 0;
     bool want_cfl = true;
     int row0 = 0, nrows = -1;  // a band of tile rows (one substep)
+    const LoopForm* loop = nullptr;  // the looping form, null: a CTA per task
+    unsigned loop_ctas = 0;
 };
+
+int set_loop_form(fv_sim* s, const KEntry* e, LoopForm* f) {
+    int per_sm = 0;
+    FV_CK(allow_smem_of(e->fn.loop, entry_smem(*e)));
+    FV_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(e->fn.loop), e->NT,
+                                                        entry_smem(*e)));
+    FV_TRY(encode_maps(s, *e, f->tmap));
+    f->grid = dim3((s->nx + e->W - 1) / e->W, (s->ny + e->H - 1) / e->H);
+    f->resident = (unsigned)(per_sm * s->ctx->sm_count);
+    f->ke = e;
+    return FV_OK;
+}
+
+// The looping form of the next run and its CTAs, where others share the GPU;
+// *form null: a CTA per task, for a simulation that runs alone, where that is
+// faster (1024 x 1024 21.5 us per step instead of 28), and for grids that fill
+// the GPU by themselves.
+//
+// A simulation takes its share of the CTAs that the GPU holds, at most 1.2 times
+// its tiles (stage_smem).  If its share is less, its speed depends on the work
+// that all do, and a tile with short chains gives way to the one of the same
+// scheme with less halo or more cells per thread (28 x 28, unsplit 60 x 28, by
+// 128 threads).  us per step and simulation, 8 threads: EE2D 200 x 600 10.0 with
+// its 12 x 12 tile, 7.0; LxF 512 x 512 4.4 with a CTA per task, 1.5.  Half and
+// twice the share: KP07_dimsplit 1024 x 1024 25.4, 20.0, FORCE 777 x 1333 9.3,
+// 6.9, EE2D 7.2, 9.0.
+int loop_form(fv_sim* s, const LoopForm** form, unsigned* ctas) {
+    *form = nullptr;
+    const int running = s->ctx->running.load(std::memory_order_relaxed);
+    if (running < 2) return FV_OK;
+    if (!s->loop.ke) {
+        FV_TRY(set_loop_form(s, s->ke, &s->loop));
+        const int w = s->ke->split ? 28 : 60;
+        for (const KEntry& e : kTable)
+            if (s->p.variant == 0 && e.scheme == s->scheme && e.W == w && e.H == 28 && e.NT == 128 &&
+                (s->ke->split ? s->ke->W < w : s->ke->W == w && s->ke->NT > 128))
+                FV_TRY(set_loop_form(s, &e, &s->wide));
+    }
+    auto wanted = [](const LoopForm& f) { return (f.grid.x * f.grid.y * 6 + 4) / 5; };
+    const LoopForm* f = &s->loop;
+    if (s->wide.ke && wanted(*f) > f->resident / running) f = &s->wide;
+    if (2 * f->grid.x * f->grid.y > 3 * f->resident) return FV_OK;
+    *form = f;
+    *ctas = std::max(1u, std::min(wanted(*f), f->resident / running));
+    return FV_OK;
+}
+
+// Tasks of a launch of a chain: 2^27 cell updates, a millisecond or less, which
+// is what other streams wait for at most.  20 steps of a 256 x 256 grid beside a
+// 4096 x 4096 one: 3.2 ms with a launch per substep, 25.5 in launches of 100
+// steps, 1.1 in chains; 0.5 in chains of an eighth of the size, which cost LxF
+// 3 % on 4096 x 4096.
+long long chain_tasks(const fv_sim* s) { return (1 << 27) / (s->ke->W * s->ke->H); }
+
+// Steps of a run in the looping form: 2^24 cell updates, after which a run takes
+// the share of the then current number of simulations (a quarter of them loses
+// 5 % at 1024 x 1024, four times as many gains nothing).
+long long loop_steps(const fv_sim* s, const LoopForm& f) {
+    return std::max<long long>(1, (1 << 24) / ((long long)f.grid.x * f.grid.y * f.ke->W * f.ke->H * s->num_substeps));
+}
 
 int launch_stage(fv_sim* s, const StagePlan& p) {
     NvtxRange range(p.nrows >= 0 ? "fv stage launch (band)" : "fv stage launch");
@@ -854,22 +962,39 @@ int launch_stage(fv_sim* s, const StagePlan& p) {
     for (int i = 0; i < p.n_tail; ++i) a.tail[i] = p.tail[i];
     a.want_cfl = p.want_cfl ? 1 : 0;
     void* kargs[] = {&a};
-    FV_CK(launch_dependent(reinterpret_cast<const void*>(s->ke->fn), dim3(tiles * (unsigned)p.n_sub), dim3(s->ke->NT),
-                           kargs, p.n_sub > 1 ? s->smem : entry_smem(*s->ke), s->stream));
-    ++s->launches;
+    if (p.loop) {
+        memcpy(a.tmap, p.loop->tmap, sizeof(a.tmap));
+        a.tiles_x = (int)p.loop->grid.x;
+        a.tiles_y = (int)p.loop->grid.y;
+        FV_CK(launch_dependent(reinterpret_cast<const void*>(p.loop->ke->fn.loop), dim3(p.loop_ctas),
+                               dim3(p.loop->ke->NT), kargs, entry_smem(*p.loop->ke), s->stream));
+        ++s->launches;
+    } else {
+        const long long most = p.n_sub > 1 ? chain_tasks(s) : tiles;
+        for (long long left = (long long)tiles * p.n_sub; left > 0;) {
+            const unsigned ctas = (unsigned)std::min(left, most);
+            left -= ctas;
+            a.followed = left > 0 ? 1 : 0;
+            FV_CK(launch_dependent(reinterpret_cast<const void*>(s->ke->fn.once), dim3(ctas), dim3(s->ke->NT), kargs,
+                                   p.n_sub > s->num_substeps ? s->smem : entry_smem(*s->ke), s->stream));
+            a.follows = 1;
+            ++s->launches;
+        }
+    }
     s->ctl_known = false;
     return FV_OK;
 }
 
-// k steps in as few launches as the grid size allows: the last n_tail of them
-// take the time steps tail[], the others the control block's dt.
+// k steps: the last n_tail of them take the time steps tail[], the others the
+// control block's dt.
 int run_steps(fv_sim* s, long long k, const float* tail, int n_tail, bool want_cfl) {
     NvtxRange range("fv steps");
-    const long long most = std::max<long long>(1, INT_MAX / ((long long)s->grid.x * s->grid.y * s->num_substeps));
+    const long long most = INT_MAX / ((long long)s->grid.x * s->grid.y * s->num_substeps);
     long long full = k - n_tail;
     while (k > 0) {
         StagePlan p;
-        p.steps = (int)std::min(k, most);
+        FV_TRY(loop_form(s, &p.loop, &p.loop_ctas));
+        p.steps = (int)std::min(k, p.loop ? loop_steps(s, *p.loop) : std::max<long long>(1, most));
         p.n_sub = p.steps * s->num_substeps;
         p.explicit_dt = false;
         p.full_steps = (int)std::min<long long>(full, p.steps);
@@ -917,12 +1042,7 @@ int fv_context_create(int device, fv_context** out) {
     auto allow_smem = [&](const KEntry& e) {
         // up to the shared memory that keeps one CTA per SM (stage_smem)
         const size_t most = std::max(entry_smem(e), (prop.sharedMemPerMultiprocessor / 2 + 127) / 128 * 128);
-        cudaError_t r = cudaFuncSetAttribute(reinterpret_cast<const void*>(e.fn),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (r == cudaSuccess)
-            r = cudaFuncSetAttribute(reinterpret_cast<const void*>(e.fn),
-                                     cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        return r;
+        return allow_smem_of(e.fn.once, most);
     };
     for (int i = 0; i < kNumEntries; ++i) FV_CK(allow_smem(kTable[i]));
     for (int i = 0; i < kNumVariants; ++i) FV_CK(allow_smem(kVariantTable[i].k));
@@ -1082,19 +1202,9 @@ int fv_sim_create(fv_context* ctx, int scheme, int nx, int ny, float dx, float d
     // kernel arguments and TMA descriptors
     StageArgs& a = s->args;
     memset(&a, 0, sizeof(StageArgs));
-    auto enc = encode_fn();
     for (int b = 0; b < 2; ++b)
-        for (int v = 0; v < nv; ++v) {
-            a.buf[b][v] = s->buf[b][v];
-            cuuint64_t dims[2] = {(cuuint64_t)(nx + 8), (cuuint64_t)(ny + 4)};
-            cuuint64_t strides[1] = {(cuuint64_t)s->pitch * sizeof(float)};
-            cuuint32_t box[2] = {(cuuint32_t)entry_box_w(*ke), (cuuint32_t)(ke->H + 4)};
-            cuuint32_t estr[2] = {1, 1};
-            CUresult r = enc(&a.tmap[b][v], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, s->buf[b][v], dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return cleanup(fail(FV_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r));
-        }
+        for (int v = 0; v < nv; ++v) a.buf[b][v] = s->buf[b][v];
+    if (encode_maps(s, *ke, a.tmap) != FV_OK) return cleanup(FV_ERR_CUDA);
     a.ctl = s->ctl;
     a.block_cfl = s->block_cfl;
     a.ticket = reinterpret_cast<unsigned*>(base + off_done);
@@ -1175,6 +1285,7 @@ int fv_sim_step(fv_sim* s, float dt) {
 int fv_sim_simulate(fv_sim* s, double t, float dt, int use_dt) {
     NvtxRange range("fv_sim_simulate");
     FV_TRY(check_sim(s));
+    const Running running(s->ctx);
     FV_TRY(read_ctl(s));
     s->ctl_known = false;  // changed below, and not uploaded if t_end is reached already
     SimCtl& c = *s->ctl_h;
@@ -1220,6 +1331,7 @@ int fv_sim_simulate(fv_sim* s, double t, float dt, int use_dt) {
 int fv_sim_advance(fv_sim* s, long long n_steps) {
     FV_TRY(check_sim(s));
     if (n_steps < 0) return fail(FV_ERR_INVALID, "negative step count");
+    const Running running(s->ctx);
     FV_TRY(read_ctl(s));
     SimCtl& c = *s->ctl_h;
     c.t_end = INFINITY;
@@ -1227,10 +1339,15 @@ int fv_sim_advance(fv_sim* s, long long n_steps) {
     host_dt_update(s);
     FV_TRY(write_ctl(s));
     FV_CK(cudaEventRecord(s->ev0, s->stream));
-    // one launch per dt interval: the end of one sets the next one's dt
+    // run by run to the next dt update: the end of one sets the next one's dt
     long long nt = c.nt;
     for (long long left = n_steps; left > 0;) {
-        const long long k = std::min(left, 100 - nt % 100);
+        long long k = std::min(left, 100 - nt % 100);
+        // A chain of launches needs a finite dt.
+        if (k * s->num_substeps * s->grid.x * s->grid.y > chain_tasks(s)) {
+            FV_TRY(read_ctl(s));
+            if (!std::isfinite(c.dt)) k = left = 1;  // no step follows it: t is not finite either
+        }
         FV_TRY(run_steps(s, k, nullptr, 0, (nt + k) % 100 == 0));
         left -= k;
         nt += k;

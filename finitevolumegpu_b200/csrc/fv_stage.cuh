@@ -79,7 +79,7 @@ struct StageArgs {
     SimCtl* ctl;
     float* block_cfl;    // one float per tile
     unsigned* ticket;    // tasks taken (launches of several substeps); zero between launches
-    unsigned* done;      // per tile, kDoneStride apart: substeps of this launch completed; zero between launches
+    unsigned* done;      // per tile, kDoneStride apart: substeps of this run completed; zero between runs
     int nx, ny, pitch;   // pitch in floats
     int tiles_x, tiles_y;
     float dx, dy, g, gamma, theta;
@@ -88,9 +88,9 @@ struct StageArgs {
     int bc;
     int order;           // RK order (KP07)
     int substeps;        // substeps (sweep orders of the split schemes, RK stages of KP07) per step
-    int first_substep;   // substep of the step that this launch starts with
-    int n_sub;           // substeps of this launch
-    int steps;           // steps this launch completes (0: a substep by itself, t and nt stay)
+    int first_substep;   // substep of the step that the run starts with
+    int n_sub;           // substeps of the run: of this launch, or of a chain of them (follows, followed)
+    int steps;           // steps the run completes (0: a substep by itself, t and nt stay)
     int full_steps;      // steps that take the control block's dt; the ones after take tail[]
     float tail[kTailSteps];
     int explicit_dt;     // all steps take dt_step, whatever the control block says
@@ -98,6 +98,8 @@ struct StageArgs {
     int want_cfl;        // compute the CFL minimum of the last substep's state
     int wait_limit;      // bounded waits: 0 = kWaitPolls polls (the default, also for zero-filled
                          // arguments), n > 0 = n polls, negative = give up at once (tests)
+    int follows;         // this launch goes on where the one before stopped in the same run of substeps
+    int followed;        // and the next one goes on where this one stops
     int tile_row0;       // first tile row of this launch (one substep may be split into launches by rows)
     int ntiles_total;    // tiles of the whole substep, 0 = this launch's; the last of them to
                          // arrive, over all launches, finishes the launch
@@ -179,13 +181,30 @@ static_assert(offsetof(SimCtl, t_end) == 8 && offsetof(SimCtl, nt) == 16 && offs
                   offsetof(SimCtl, update_dt) == 40 && offsetof(SimCtl, cur) == 44,
               "the vector loads of control blocks follow SimCtl's layout");
 
-template <int NT>
-__device__ __forceinline__ float block_min(float v, float* red) {
+// A value that the compiler takes for a new one in every task of a looping
+// kernel: what follows from it is computed per task instead of being kept in
+// registers from task to task.
+template <bool LOOP, class T>
+__device__ __forceinline__ T per_task(T v) {
+    if constexpr (LOOP && std::is_same<T, float>::value) asm volatile("" : "+f"(v));
+    else if constexpr (LOOP) asm volatile("" : "+r"(v));
+    return v;
+}
+
+// The thread's index in its CTA; tid, from per_task, in a looping kernel.
+template <bool LOOP>
+__device__ __forceinline__ unsigned thread_of(unsigned tid) {
+    if constexpr (LOOP) return tid;
+    else return threadIdx.x;
+}
+
+template <int NT, bool LOOP = false>
+__device__ __forceinline__ float block_min(float v, float* red, unsigned tid) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5;
+    const int w = thread_of<LOOP>(tid) >> 5;
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[w] = v;
+    if ((thread_of<LOOP>(tid) & 31) == 0) red[w] = v;
     __syncthreads();
     float r = red[0];
 #pragma unroll
@@ -216,21 +235,22 @@ struct TileJob {
     float* const* out;        // NV output planes
     int nx, ny, pitch, bc;
     int x0, y0;               // first interior cell of the tile
+    unsigned tid;             // thread of the CTA (per_task)
 };
 
 // Issues the TMA loads of the tile (thread 0) and waits for them with a bounded
 // wait of `polls` polls on `phase` of the mbarrier (initialised here when
 // `init`).  Returns false (uniformly across the CTA) if the wait gave up; *err
 // is then set, after a second bounded wait has let the copies in flight land.
-template <int NV, int SP, int TR>
+template <int NV, int SP, int TR, bool LOOP>
 __device__ __forceinline__ bool load_tile(float* Qs, const CUtensorMap* tmap, int x0, int y0, uint64_t* bar,
-                                          uint32_t phase, bool init, int* err, uint32_t polls = kWaitPolls) {
+                                          uint32_t phase, bool init, unsigned tid, int* err, uint32_t polls = kWaitPolls) {
     constexpr int PS = SP * TR;
     // Each variable's plane is the destination of a tensor copy, which must
     // start on a 128-byte boundary: tiles whose (W+8) x (H+4) plane is not a
     // multiple of 32 floats would misalign every plane after the first.
     static_assert((PS * sizeof(float)) % 128 == 0, "variable planes in shared memory must be 128-byte aligned");
-    if (threadIdx.x == 0) {
+    if (thread_of<LOOP>(tid) == 0) {
         if (init) {
             mbar_init(bar, 1);
             fence_barrier_init();
@@ -247,7 +267,7 @@ __device__ __forceinline__ bool load_tile(float* Qs, const CUtensorMap* tmap, in
     const bool ok = mbar_wait_bounded(bar, phase, polls);
     const int failed = __syncthreads_or(ok ? 0 : 1);
     if (failed) {
-        if (threadIdx.x == 0) atomicExch(err, 1);
+        if (thread_of<LOOP>(tid) == 0) atomicExch(err, 1);
         mbar_wait_bounded(bar, phase, kWaitPolls);  // let copies in flight land before the CTA moves on
         return false;
     }
@@ -297,7 +317,7 @@ __device__ __forceinline__ float sign_y(int v) { return v == 2 ? -1.0f : 1.0f; }
 // wrapped cell from global memory, then reflective sides mirror interior cells
 // with the normal momentum negated, north, south, east, west in turn.
 // Dirichlet ghosts keep the stored values the TMA load brought in.
-template <int NV, int W, int H, int NT, int SP = W + 8>
+template <int NV, int W, int H, int NT, int SP, bool LOOP>
 __device__ void apply_boundary(float* Qs, const TileJob& J) {
     constexpr int TR = H + 4, PS = SP * TR;
     const int nx = J.nx, ny = J.ny, bc = J.bc, x0 = J.x0, y0 = J.y0;
@@ -318,7 +338,7 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
         const int lo_c = (pw && x0 == 0) ? 2 : 0, hi_c = pe ? max(0, min(2, SP - col_e)) : 0;
         const int in_rows = (lo_r + hi_r) * SP, all = in_rows + (lo_c + hi_c) * TR;
 #pragma unroll 4
-        for (int i = threadIdx.x; i < all; i += NT) {
+        for (int i = thread_of<LOOP>(J.tid); i < all; i += NT) {
             int t, s;
             bool use = true;
             if (i < in_rows) {
@@ -345,7 +365,7 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
     }
     // Tile row of domain row y: t = y - y0 + 2; tile column of x: s = x - x0 + 4.
     if (bc_north(bc) == BC_REFLECTIVE && y0 + H + 2 > ny) {
-        for (int i = threadIdx.x; i < 2 * SP; i += NT) {
+        for (int i = thread_of<LOOP>(J.tid); i < 2 * SP; i += NT) {
             const int m = i / SP, s = i - m * SP;
             const int t = ny + m - y0 + 2, ts = ny - 1 - m - y0 + 2;
             if (t < TR) {
@@ -356,7 +376,7 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
         __syncthreads();
     }
     if (bc_south(bc) == BC_REFLECTIVE && y0 == 0) {
-        for (int i = threadIdx.x; i < 2 * SP; i += NT) {
+        for (int i = thread_of<LOOP>(J.tid); i < 2 * SP; i += NT) {
             const int m = i / SP, s = i - m * SP;
             const int t = -1 - m + 2, ts = m + 2;
             if (ts < TR) {
@@ -367,7 +387,7 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
         __syncthreads();
     }
     if (bc_east(bc) == BC_REFLECTIVE && x0 + W + 2 > nx) {
-        for (int i = threadIdx.x; i < 2 * TR; i += NT) {
+        for (int i = thread_of<LOOP>(J.tid); i < 2 * TR; i += NT) {
             const int m = i / TR, t = i - m * TR;
             const int s = nx + m - x0 + 4, ss = nx - 1 - m - x0 + 4;
             if (s < SP) {
@@ -378,7 +398,7 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
         __syncthreads();
     }
     if (bc_west(bc) == BC_REFLECTIVE && x0 == 0) {
-        for (int i = threadIdx.x; i < 2 * TR; i += NT) {
+        for (int i = thread_of<LOOP>(J.tid); i < 2 * TR; i += NT) {
             const int m = i / TR, t = i - m * TR;
             const int s = -1 - m + 4, ss = m + 4;
             if (ss < SP) {
@@ -695,12 +715,22 @@ __device__ __forceinline__ void walk_line2(float* line, int step, int d2, int a,
     }
 }
 
+// Sets a walker's prefetched cells where it has none.  In a looping kernel they
+// would otherwise count as kept from the last task, a register each.
+template <class N, int M, int NV>
+__device__ __forceinline__ void clear(N (&pre)[M][NV]) {
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) pre[m][v] = splat<N>(0.0f);
+}
+
 // x sweep over tile rows [t0, t1): interior columns updated in place.
 // LPT = 2: a thread walks rows t and t + (t1 - t0)/2 side by side.
-template <int SCHEME, int NV, int W, int H, int NT, int VAR, int LPT>
-__device__ __forceinline__ void sweep_x(float* Qs, int t0, int t1, const SweepPar& p) {
+template <int SCHEME, int NV, int W, int H, int NT, int VAR, int LPT, bool LOOP>
+__device__ __forceinline__ void sweep_x(float* Qs, unsigned tid, int t0, int t1, const SweepPar& p) {
     constexpr int SP = split_pitch(W), PS = SP * (H + 4), NSEG = split_nseg_x(W), R = W / NSEG;
-    const int item = threadIdx.x;
+    const int item = thread_of<LOOP>(tid);
     const int nlines = (t1 - t0) / LPT;
     const bool has = item < nlines * NSEG;
     const int t = t0 + item / NSEG, seg = item % NSEG;
@@ -714,6 +744,9 @@ __device__ __forceinline__ void sweep_x(float* Qs, int t0, int t1, const SweepPa
             ld_cell<NV, false, PS>(line, b, 1, pre[2]);
             ld_cell<NV, false, PS>(line, b + 1, 1, pre[3]);
         }
+        if constexpr (LOOP) {
+            if (!has) clear(pre);
+        }
         __syncthreads();
         if (has) walk_line<SCHEME, false, PS, VAR>(line, 1, a, b, pre, p);
     } else {
@@ -725,6 +758,9 @@ __device__ __forceinline__ void sweep_x(float* Qs, int t0, int t1, const SweepPa
             ld_cell<NV, false, PS>(line, b, 1, d2, pre[2]);
             ld_cell<NV, false, PS>(line, b + 1, 1, d2, pre[3]);
         }
+        if constexpr (LOOP) {
+            if (!has) clear(pre);
+        }
         __syncthreads();
         if (has) walk_line2<SCHEME, false, PS, VAR>(line, 1, d2, a, b, pre, p);
     }
@@ -733,12 +769,12 @@ __device__ __forceinline__ void sweep_x(float* Qs, int t0, int t1, const SweepPa
 
 // y sweep over tile columns [s0, s1): interior rows updated in place.
 // LPT = 2: a thread walks columns s and s + (s1 - s0)/2 side by side.
-template <int SCHEME, int NV, int W, int H, int NT, int VAR, int LPT>
-__device__ __forceinline__ void sweep_y(float* Qs, int s0, int s1, const SweepPar& p) {
+template <int SCHEME, int NV, int W, int H, int NT, int VAR, int LPT, bool LOOP>
+__device__ __forceinline__ void sweep_y(float* Qs, unsigned tid, int s0, int s1, const SweepPar& p) {
     constexpr int SP = split_pitch(W), PS = SP * (H + 4);
     constexpr int NSEG = NT * LPT / (W + 4), R = H / NSEG;
     const int ncols = (s1 - s0) / LPT;
-    const int item = threadIdx.x;
+    const int item = thread_of<LOOP>(tid);
     const bool has = item < ncols * NSEG;
     const int s = s0 + item % ncols, seg = item / ncols;
     const int a = 2 + seg * R, b = a + R;
@@ -751,6 +787,9 @@ __device__ __forceinline__ void sweep_y(float* Qs, int s0, int s1, const SweepPa
             ld_cell<NV, true, PS>(line, b, SP, pre[2]);
             ld_cell<NV, true, PS>(line, b + 1, SP, pre[3]);
         }
+        if constexpr (LOOP) {
+            if (!has) clear(pre);
+        }
         __syncthreads();
         if (has) walk_line<SCHEME, true, PS, VAR>(line, SP, a, b, pre, p);
     } else {
@@ -761,6 +800,9 @@ __device__ __forceinline__ void sweep_y(float* Qs, int s0, int s1, const SweepPa
             ld_cell<NV, true, PS>(line, a - 1, SP, d2, pre[1]);
             ld_cell<NV, true, PS>(line, b, SP, d2, pre[2]);
             ld_cell<NV, true, PS>(line, b + 1, SP, d2, pre[3]);
+        }
+        if constexpr (LOOP) {
+            if (!has) clear(pre);
         }
         __syncthreads();
         if (has) walk_line2<SCHEME, true, PS, VAR>(line, SP, d2, a, b, pre, p);
@@ -786,7 +828,8 @@ struct SplitPar {
 // instead of the TMA (bar, phase, init_bar, err and polls are then unused).
 // HEALTH (batched kernels): with `health` set, *unhealthy becomes true if any
 // written cell holds a non-finite value or a non-positive depth (density).
-template <int SCHEME, int W, int H, int NT, bool ASYNC_LOAD = false, int VAR = 0, int LPT = 1, bool HEALTH = false>
+template <int SCHEME, int W, int H, int NT, bool ASYNC_LOAD = false, int VAR = 0, int LPT = 1, bool HEALTH = false,
+          bool LOOP = false>
 __device__ bool process_tile_dimsplit(float* Qs, uint64_t* bar, uint32_t phase, bool init_bar, const TileJob& J,
                                       const SplitPar& P, bool do_cfl, int* err, float& my_cfl,
                                       uint32_t polls = kWaitPolls, bool health = false, bool* unhealthy = nullptr) {
@@ -805,10 +848,10 @@ __device__ bool process_tile_dimsplit(float* Qs, uint64_t* bar, uint32_t phase, 
     if constexpr (ASYNC_LOAD) {
         load_tile_async<NV, SP, TR, NT>(Qs, J);
     } else {
-        if (!load_tile<NV, SP, TR>(Qs, J.tmap, J.x0, J.y0, bar, phase, init_bar, err, polls)) return false;
+        if (!load_tile<NV, SP, TR, LOOP>(Qs, J.tmap, J.x0, J.y0, bar, phase, init_bar, J.tid, err, polls)) return false;
     }
     const int x0 = J.x0, y0 = J.y0;
-    if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<NV, W, H, NT, SP>(Qs, J);
+    if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<NV, W, H, NT, SP, LOOP>(Qs, J);
 
     SweepPar p;
     p.theta = P.theta;
@@ -821,14 +864,14 @@ __device__ bool process_tile_dimsplit(float* Qs, uint64_t* bar, uint32_t phase, 
     const bool x_first = (SCHEME == FORCE || SCHEME == HLL) ? true : (P.substep == 0);
     if (x_first) {
         p.set_direction(P.dx);
-        sweep_x<SCHEME, NV, W, H, NT, VAR, LPT>(Qs, 2 - G, H + 2 + G, p);
+        sweep_x<SCHEME, NV, W, H, NT, VAR, LPT, LOOP>(Qs, J.tid, 2 - G, H + 2 + G, p);
         p.set_direction(P.dy);
-        sweep_y<SCHEME, NV, W, H, NT, VAR, LPT>(Qs, 4, W + 4, p);
+        sweep_y<SCHEME, NV, W, H, NT, VAR, LPT, LOOP>(Qs, J.tid, 4, W + 4, p);
     } else {
         p.set_direction(P.dy);
-        sweep_y<SCHEME, NV, W, H, NT, VAR, LPT>(Qs, 4 - G, W + 4 + G, p);
+        sweep_y<SCHEME, NV, W, H, NT, VAR, LPT, LOOP>(Qs, J.tid, 4 - G, W + 4 + G, p);
         p.set_direction(P.dx);
-        sweep_x<SCHEME, NV, W, H, NT, VAR, LPT>(Qs, 2, H + 2, p);
+        sweep_x<SCHEME, NV, W, H, NT, VAR, LPT, LOOP>(Qs, J.tid, 2, H + 2, p);
     }
 
     // copy-out of the interior (+ gravity source, CFL); the output plane
@@ -839,7 +882,7 @@ __device__ bool process_tile_dimsplit(float* Qs, uint64_t* bar, uint32_t phase, 
     float* outp[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) outp[v] = J.out[v];
-    for (int i = threadIdx.x; i < H * QW; i += NT) {
+    for (int i = thread_of<LOOP>(J.tid); i < H * QW; i += NT) {
         const int r = i / QW, q = i - r * QW;
         const int y = y0 + r, x = x0 + 4 * q;
         if (y >= J.ny || x >= J.nx) continue;
@@ -953,7 +996,7 @@ struct UnsplitPar {
 // ASYNC_LOAD (batched kernels): the tile comes in through load_tile_async.
 // HEALTH (batched kernels): with `health` set, *unhealthy becomes true if a
 // written cell holds a non-finite value or a non-positive depth.
-template <int SCHEME, int W, int H, int NT, bool ASYNC_LOAD = false, bool HEALTH = false>
+template <int SCHEME, int W, int H, int NT, bool ASYNC_LOAD = false, bool HEALTH = false, bool LOOP = false>
 __device__ bool process_tile_unsplit(float* Qs, uint64_t* bar, uint32_t phase, bool init_bar, const TileJob& J,
                                      const UnsplitPar& P, bool do_cfl, int* err, float& my_cfl,
                                      uint32_t polls = kWaitPolls, bool health = false, bool* unhealthy = nullptr) {
@@ -966,17 +1009,17 @@ __device__ bool process_tile_unsplit(float* Qs, uint64_t* bar, uint32_t phase, b
     if constexpr (ASYNC_LOAD) {
         load_tile_async<3, SP, TR, NT>(Qs, J);
     } else {
-        if (!load_tile<3, SP, TR>(Qs, J.tmap, x0, y0, bar, phase, init_bar, err, polls)) return false;
+        if (!load_tile<3, SP, TR, LOOP>(Qs, J.tmap, x0, y0, bar, phase, init_bar, thread_of<LOOP>(J.tid), err, polls)) return false;
     }
     {
-        if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<3, W, H, NT>(Qs, J);
+        if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<3, W, H, NT, SP, LOOP>(Qs, J);
         const float kdt = P.kdt;
         const float g = P.g, half_g = fmul(0.5f, g), theta2 = minmod_theta2(P.theta);
         const float k4x = fdiv_fast(P.dx, fmul(4.0f, kdt)), k4y = fdiv_fast(P.dy, fmul(4.0f, kdt));
         const float kdx = fdiv_fast(kdt, P.dx), kdy = fdiv_fast(kdt, P.dy);
         const bool blend = (SCHEME == KP07) && P.order == 2 && P.substep == 1;
 
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int warp = thread_of<LOOP>(J.tid) >> 5, lane = thread_of<LOOP>(J.tid) & 31;
         const int wx = warp % WX, seg = warp / WX;
         const int s = 3 + 30 * wx + lane;  // tile column of this lane
         const int x = x0 + s - 4;          // domain column
@@ -1163,9 +1206,9 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
     return scheme == LXF || scheme == FORCE || scheme == HLL || (scheme == WAF && W != 60) ? 1 : 0;
 }
 
-// Stage kernel of any scheme.  A launch has one CTA per tile and substep.
+// Stage kernel of any scheme, with one CTA per task, a tile in one substep.
 //
-// A launch of one substep takes its tiles by block index.  A launch of several
+// A launch of one substep takes its tiles by block index.  A run of several
 // substeps has no barrier between them: a CTA takes the next task, in the order
 // substep by substep and row by row of tiles, and waits until the tiles within
 // two cells of its own have completed the substep before, which is all that it
@@ -1173,7 +1216,30 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
 // order in which CTAs start and depend on earlier ones only, so whatever part of
 // the grid is resident makes progress; nothing needs the grid to be resident at
 // once.  The waits are bounded: a CTA that gives up sets the error flag, and the
-// launch then runs to its end with the state left undefined.
+// run then goes on to its end with the state left undefined.
+//
+// A long run is a chain of launches, so that work of other streams gets its
+// turn between them (chain_tasks).  They share the task and progress counters
+// and start wherever in a substep the one before stopped.  A launch starts as
+// soon as the one before has handed out its tasks; instead of the end of that
+// one it waits for the tiles that it reads, as within a launch, so the chain has
+// no gaps: KP07_dimsplit 4096 x 4096 in one launch per 100 steps, in a chain of
+// 18, and in 17 launches that each wait for the end of the one before: 260.8,
+// 261.1 and 265.6 us per step; LxF 84.4, 84.7 and 105.7.  Its CTAs end after the
+// launch before has ended, so the end of the last launch is that of the run.
+//
+// LOOP: the form for GPUs shared with other simulations of the context.  The
+// launch has fewer CTAs than tasks (loop_form) and each takes task after task,
+// so that none is queued behind others and simulations run beside each other.
+// us per step and simulation with 1, 2, 4 and 8 threads that each run one:
+//                             a launch per substep    CTA per task            LOOP from 2 on
+//   KP07_dimsplit 64 x 48     14.7  7.8  4.0  2.1     7.7  7.3  7.3  7.2      7.7  4.4  2.0  1.2
+//   KP07_dimsplit 256 x 256   16.1  8.4  4.7  3.3     10.2 9.7  9.8  9.7      10.0 6.1  3.8  3.0
+//   FORCE 777 x 1333          14.4  9.3  6.0  6.3     8.1  7.7  7.7  7.6      8.1  6.9  6.7  6.9
+//   KP07_dimsplit 1024 x 1024 35.6 26.8 19.8 19.7     21.8 21.4 21.3 21.3     21.7 21.3 19.8 20.1
+// A CTA keeps nothing but its task between two of them (per_task, clear): with
+// what the compiler would keep, KP07_dimsplit's 28 x 28 tile takes 128 registers
+// instead of 71.
 //
 // Against one launch per substep this fills the tail of a substep with the next
 // one's tiles, lets tile loads overlap other tiles' sweeps where a substep is
@@ -1190,7 +1256,7 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
 //   KP07_dimsplit  15.1  10.5   9.9    34.5  22.0  21.7   84.7  67.3  66.5    282   264   261
 //   EE2D           18.4  13.5  10.0    46.5  31.1  29.6    128   109   104    440   422   403
 // (FORCE before and now: 6.5 3.4, 13.3 8.0, 35.3 26.6, 111 105).
-template <int SCHEME, int W, int H, int NT, int VAR = 0, int LPT = 1>
+template <int SCHEME, int W, int H, int NT, int VAR = 0, int LPT = 1, bool LOOP = false>
 __global__ void __launch_bounds__(NT, compiled_blocks(SCHEME, W, H, NT, LPT)) stage_kernel(const __grid_constant__ StageArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* Qs = reinterpret_cast<float*>(smem_raw);
@@ -1199,19 +1265,23 @@ __global__ void __launch_bounds__(NT, compiled_blocks(SCHEME, W, H, NT, LPT)) st
     __shared__ float red[NT / 32];
     __shared__ int am_last;
 
-    grid_dependency_wait();  // the previous launch's state, control block and counters
+    if (LOOP || !A.follows) grid_dependency_wait();  // the previous launch's state, control block and counters
+    // The control block changes when the run's last task is complete.  A looping
+    // CTA may start later than that: it takes its ticket after these loads, and
+    // then finds no task left.
     const int4 w0 = ld_relaxed_v4(A.ctl);                                      // t, t_end
     const int4 w1 = ld_relaxed_v4(reinterpret_cast<const char*>(A.ctl) + 16);  // nt, dt, cfl_min
     const int4 w2 = ld_relaxed_v4(reinterpret_cast<const char*>(A.ctl) + 32);  // factor, cfl_scale, update_dt, cur
     const float dt0 = A.explicit_dt ? A.dt_step : __int_as_float(w1.z);
     const int cur0 = w2.w;
     int n_sub = A.n_sub, steps = A.steps;
-    bool want_cfl = A.want_cfl != 0;
+    bool want_cfl = A.want_cfl != 0, active = true;
     if (!A.explicit_dt) {
         // a step runs while t < t_end and dt > 0 (GPUSimulators/Simulator.py:192, :202);
         // a dt that is not finite takes t past any end time in one step
         const double t = __hiloint2double(w0.y, w0.x), t_end = __hiloint2double(w0.w, w0.z);
-        if (!(t < t_end) || dt0 <= 0.0f) return;
+        active = t < t_end && !(dt0 <= 0.0f);
+        if (!LOOP && !active) return;
         if (A.full_steps > 0 && !(fabsf(dt0) < __int_as_float(0x7f800000))) {
             n_sub = A.substeps;
             steps = 1;
@@ -1219,119 +1289,176 @@ __global__ void __launch_bounds__(NT, compiled_blocks(SCHEME, W, H, NT, LPT)) st
         }
     }
     const int ntiles = A.tiles_x * A.tiles_y;
+    // Substeps that have tasks.  The looping form keeps those of substeps past
+    // n_sub, without work: the control block changes after the last task only.
+    const int n_all = LOOP ? A.n_sub : n_sub;
     unsigned task = blockIdx.x;
     if (A.n_sub > 1) {
-        if (task >= (unsigned)ntiles * (unsigned)n_sub) return;
+        if (!LOOP && task >= (unsigned)ntiles * (unsigned)n_sub) return;
+        if (threadIdx.x == 0) taken = atomicAdd(A.ticket, 1u);
+        __syncthreads();
+        task = taken;
+        if (!LOOP && A.followed) grid_launch_dependents();
+    }
+    uint32_t loads = 0;   // tile loads of this CTA
+    bool broken = false;  // one of them gave up
+
+    while (!LOOP || (active && task < (unsigned)ntiles * (unsigned)n_all)) {
+        const unsigned tid = per_task<LOOP>(threadIdx.x);
+        if (LOOP) __builtin_assume(tid < NT);
+        const unsigned row = task / (unsigned)A.tiles_x;
+        const int tx = (int)(task - row * (unsigned)A.tiles_x);
+        const int s = A.n_sub > 1 ? (int)(row / (unsigned)A.tiles_y) : 0;
+        const int ty = (int)row - s * A.tiles_y + A.tile_row0;
+
+        bool ok = true;
+        if (s > 0 && tid < 16) {
+            const int i = tid & 3, j = tid >> 2;
+            const bool wrap_x = bc_west(A.bc) == BC_PERIODIC || bc_east(A.bc) == BC_PERIODIC;
+            const bool wrap_y = bc_south(A.bc) == BC_PERIODIC || bc_north(A.bc) == BC_PERIODIC;
+            const int nx = near_tile(tx, i, A.nx, A.tiles_x, W, wrap_x);
+            const int ny = near_tile(ty, j, A.ny, A.tiles_y, H, wrap_y);
+            if (tid == 15 || nx != tx || ny != ty) {  // thread 15 waits for the tile itself
+                const unsigned* p = A.done + (size_t)kDoneStride * (ny * A.tiles_x + nx);
+                const uint32_t polls = wait_polls(A.wait_limit);
+                ok = false;
+                for (uint32_t k = 0; k < polls; ++k) {
+                    if (ld_acquire(p) >= (unsigned)s) {
+                        ok = true;
+                        break;
+                    }
+                    __nanosleep(20);
+                }
+            }
+        }
+        const bool run = !__syncthreads_or(ok && !(LOOP && broken) ? 0 : 1);
+        const bool last = s == n_all - 1;
+        const int sub = (A.first_substep + s) % A.substeps, step = s / A.substeps;
+        const bool do_cfl = (LOOP ? s == n_sub - 1 : last) && want_cfl && SCHEME != WAF;  // WAFKernel has no CFL output (SWE2D_WAF.cu:103-119)
+        float my_cfl = __int_as_float(0x7f800000);
+        if (run && (!LOOP || s < n_sub)) {
+            const int cur = cur0 ^ (s & 1);
+            const float dt = (A.explicit_dt || step < A.full_steps) ? dt0 : A.tail[step - A.full_steps];
+            const float kdt = dt * A.dt_scale;
+            TileJob J;
+            J.tmap = &A.tmap[cur][0];
+            J.in = A.buf[cur];
+            J.out = A.buf[cur ^ 1];
+            J.nx = per_task<LOOP>(A.nx);
+            J.ny = per_task<LOOP>(A.ny);
+            J.pitch = per_task<LOOP>(A.pitch);
+            J.bc = per_task<LOOP>(A.bc);
+            J.x0 = tx * W;
+            J.y0 = ty * H;
+            J.tid = tid;
+            // the other tiles' stores, which the wait above ordered before this
+            // point, precede the tensor copies of the tile load
+            if (tid == 0) fence_proxy_async_global();
+            const float dx = per_task<LOOP>(A.dx), dy = per_task<LOOP>(A.dy), g = per_task<LOOP>(A.g),
+                        theta = per_task<LOOP>(A.theta);
+            const uint32_t phase = LOOP ? loads & 1u : 0u;
+            const bool init = !LOOP || loads == 0;
+            bool loaded;
+            if constexpr (SCHEME == LXF || SCHEME == KP07) {
+                const UnsplitPar P{dx, dy, g, theta, kdt, sub, A.order};
+                loaded = process_tile_unsplit<SCHEME, W, H, NT, false, false, LOOP>(Qs, &bar, phase, init, J, P, do_cfl, &A.ctl->error,
+                                                                my_cfl, wait_polls(A.wait_limit));
+            } else {
+                const SplitPar P{dx, dy, g, per_task<LOOP>(A.gamma), theta, kdt, sub, per_task<LOOP>(A.variant_beta)};
+                loaded = process_tile_dimsplit<SCHEME, W, H, NT, false, VAR, LPT, false, LOOP>(
+                    Qs, &bar, phase, init, J, P, do_cfl, &A.ctl->error, my_cfl, wait_polls(A.wait_limit));
+            }
+            if (LOOP) {
+                ++loads;
+                broken = !loaded;  // its barrier's phase is not known any more: no further load
+            }
+            fence_proxy_async_global();  // these stores precede other tiles' tensor copies
+        } else if (!run && tid == 0) {
+            atomicExch(&A.ctl->error, 1);
+        }
+        const int tile = ty * A.tiles_x + tx;
+        if constexpr (LOOP) {  // (below for the others)
+            if (do_cfl) {
+                const float m = block_min<NT, true>(my_cfl, red, tid);
+                if (tid == 0) A.block_cfl[tile] = m;
+            }
+        }
+        if (!last) {
+            __syncthreads();
+            if (tid == 0) st_release(A.done + (size_t)kDoneStride * tile, (unsigned)s + 1u);
+            if constexpr (!LOOP) {
+                if (A.follows) grid_dependency_wait();
+                return;
+            }
+        } else {
+            // The last substep: CFL minimum of the tile, arrival, and in the CTA that
+            // arrives last the control-block update of Simulator.step / simulate
+            // (GPUSimulators/Simulator.py:195-196, :227-228).  The tile is written: the
+            // next launch's CTAs may start once every CTA of this one is here (they
+            // wait in grid_dependency_wait for its end).
+            if constexpr (!LOOP) {
+                grid_launch_dependents();
+                if (do_cfl) {
+                    const float m = block_min<NT>(my_cfl, red, tid);
+                    if (tid == 0) A.block_cfl[tile] = m;
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                am_last = atomicAdd(&A.ctl->arrive, 1u) == (unsigned)(A.ntiles_total ? A.ntiles_total : ntiles) - 1u;
+            }
+            __syncthreads();
+            if constexpr (!LOOP) {
+                if (A.follows) grid_dependency_wait();
+                if (!am_last) return;
+            }
+            if (!LOOP || am_last) {
+                __threadfence();
+                float m = __int_as_float(0x7f800000);
+                const bool new_cfl = LOOP ? want_cfl && SCHEME != WAF : do_cfl;
+                if (new_cfl) {
+                    for (int i = tid; i < ntiles; i += NT) m = fminf(m, __ldcg(&A.block_cfl[i]));
+                    m = block_min<NT, LOOP>(m, red, tid);
+                }
+                if (!LOOP && A.n_sub > 1)  // every task is complete: no CTA takes or polls any more
+                    for (int i = tid; i < ntiles; i += NT) A.done[(size_t)kDoneStride * i] = 0u;
+                if (tid == 0) {
+                    SimCtl* c = A.ctl;
+                    c->cur = cur0 ^ (n_sub & 1);
+                    if (new_cfl) c->cfl_min = m;
+                    if (steps > 0) {
+                        double t = c->t;
+                        for (int k = 0; k < steps; ++k)
+                            t += (double)((A.explicit_dt || k < A.full_steps) ? dt0 : A.tail[k - A.full_steps]);
+                        c->t = t;
+                        c->nt += steps;
+                        if (!A.explicit_dt && c->update_dt && (c->nt % 100 == 0)) c->dt = (c->cfl_min * c->factor) * c->cfl_scale;
+                    }
+                    c->arrive = 0u;
+                    if (!LOOP && A.n_sub > 1) *A.ticket = 0u;
+                }
+            }
+        }
+        if constexpr (!LOOP) return;
         if (threadIdx.x == 0) taken = atomicAdd(A.ticket, 1u);
         __syncthreads();
         task = taken;
     }
-    const unsigned row = task / (unsigned)A.tiles_x;
-    const int tx = (int)(task - row * (unsigned)A.tiles_x);
-    const int s = A.n_sub > 1 ? (int)(row / (unsigned)A.tiles_y) : 0;
-    const int ty = (int)row - s * A.tiles_y + A.tile_row0;
 
-    bool ok = true;
-    if (s > 0 && threadIdx.x < 16) {
-        const int i = threadIdx.x & 3, j = threadIdx.x >> 2;
-        const bool wrap_x = bc_west(A.bc) == BC_PERIODIC || bc_east(A.bc) == BC_PERIODIC;
-        const bool wrap_y = bc_south(A.bc) == BC_PERIODIC || bc_north(A.bc) == BC_PERIODIC;
-        const int nx = near_tile(tx, i, A.nx, A.tiles_x, W, wrap_x);
-        const int ny = near_tile(ty, j, A.ny, A.tiles_y, H, wrap_y);
-        if (threadIdx.x == 15 || nx != tx || ny != ty) {  // thread 15 waits for the tile itself
-            const unsigned* p = A.done + (size_t)kDoneStride * (ny * A.tiles_x + nx);
-            const uint32_t polls = wait_polls(A.wait_limit);
-            ok = false;
-            for (uint32_t k = 0; k < polls; ++k) {
-                if (ld_acquire(p) >= (unsigned)s) {
-                    ok = true;
-                    break;
-                }
-                __nanosleep(20);
-            }
-        }
-    }
-    const bool run = !__syncthreads_or(ok ? 0 : 1);
-    const bool last = s == n_sub - 1;
-    const int sub = (A.first_substep + s) % A.substeps, step = s / A.substeps;
-    const bool do_cfl = last && want_cfl && SCHEME != WAF;  // WAFKernel has no CFL output (SWE2D_WAF.cu:103-119)
-    float my_cfl = __int_as_float(0x7f800000);
-    if (run) {
-        const int cur = cur0 ^ (s & 1);
-        const float dt = (A.explicit_dt || step < A.full_steps) ? dt0 : A.tail[step - A.full_steps];
-        const float kdt = dt * A.dt_scale;
-        TileJob J;
-        J.tmap = &A.tmap[cur][0];
-        J.in = A.buf[cur];
-        J.out = A.buf[cur ^ 1];
-        J.nx = A.nx;
-        J.ny = A.ny;
-        J.pitch = A.pitch;
-        J.bc = A.bc;
-        J.x0 = tx * W;
-        J.y0 = ty * H;
-        // the other tiles' stores, which the wait above ordered before this
-        // point, precede the tensor copies of the tile load
-        if (threadIdx.x == 0) fence_proxy_async_global();
-        if constexpr (SCHEME == LXF || SCHEME == KP07) {
-            const UnsplitPar P{A.dx, A.dy, A.g, A.theta, kdt, sub, A.order};
-            process_tile_unsplit<SCHEME, W, H, NT>(Qs, &bar, 0, true, J, P, do_cfl, &A.ctl->error, my_cfl,
-                                                   wait_polls(A.wait_limit));
-        } else {
-            const SplitPar P{A.dx, A.dy, A.g, A.gamma, A.theta, kdt, sub, A.variant_beta};
-            process_tile_dimsplit<SCHEME, W, H, NT, false, VAR, LPT>(Qs, &bar, 0, true, J, P, do_cfl, &A.ctl->error,
-                                                                     my_cfl, wait_polls(A.wait_limit));
-        }
-        fence_proxy_async_global();  // these stores precede other tiles' tensor copies
-    } else if (threadIdx.x == 0) {
-        atomicExch(&A.ctl->error, 1);
-    }
-    const int tile = ty * A.tiles_x + tx;
-    if (!last) {
+    if constexpr (LOOP) {
+        // The last CTA to leave clears the counters: no CTA takes or polls any more.
+        grid_launch_dependents();
         __syncthreads();
-        if (threadIdx.x == 0) st_release(A.done + (size_t)kDoneStride * tile, (unsigned)s + 1u);
-        return;
-    }
-
-    // The last substep: CFL minimum of the tile, arrival, and in the CTA that
-    // arrives last the control-block update of Simulator.step / simulate
-    // (GPUSimulators/Simulator.py:195-196, :227-228).  The tile is written: the
-    // next launch's CTAs may start once every CTA of this one is here (they
-    // wait in grid_dependency_wait for its end).
-    grid_launch_dependents();
-    if (do_cfl) {
-        const float m = block_min<NT>(my_cfl, red);
-        if (threadIdx.x == 0) A.block_cfl[tile] = m;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        am_last = atomicAdd(&A.ctl->arrive, 1u) == (unsigned)(A.ntiles_total ? A.ntiles_total : ntiles) - 1u;
-    }
-    __syncthreads();
-    if (!am_last) return;
-    __threadfence();
-    float m = __int_as_float(0x7f800000);
-    if (do_cfl) {
-        for (int i = threadIdx.x; i < ntiles; i += NT) m = fminf(m, __ldcg(&A.block_cfl[i]));
-        m = block_min<NT>(m, red);
-    }
-    if (A.n_sub > 1)  // every task is complete: no CTA takes or polls any more
-        for (int i = threadIdx.x; i < ntiles; i += NT) A.done[(size_t)kDoneStride * i] = 0u;
-    if (threadIdx.x == 0) {
-        SimCtl* c = A.ctl;
-        c->cur = cur0 ^ (n_sub & 1);
-        if (do_cfl) c->cfl_min = m;
-        if (steps > 0) {
-            double t = c->t;
-            for (int k = 0; k < steps; ++k)
-                t += (double)((A.explicit_dt || k < A.full_steps) ? dt0 : A.tail[k - A.full_steps]);
-            c->t = t;
-            c->nt += steps;
-            if (!A.explicit_dt && c->update_dt && (c->nt % 100 == 0)) c->dt = (c->cfl_min * c->factor) * c->cfl_scale;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            am_last = atomicAdd(A.ticket + 1, 1u) == gridDim.x - 1u;
         }
-        c->arrive = 0u;
-        if (A.n_sub > 1) *A.ticket = 0u;
+        __syncthreads();
+        if (!am_last) return;
+        __threadfence();
+        for (int i = threadIdx.x; i < ntiles; i += NT) A.done[(size_t)kDoneStride * i] = 0u;
+        if (threadIdx.x < 2) A.ticket[threadIdx.x] = 0u;
     }
 }
 
@@ -1467,6 +1594,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     J.ny = I.ny;
     J.pitch = I.pitch;
     J.bc = I.bc;
+    J.tid = threadIdx.x;
     const int ty = job.y / I.tiles_x;
     J.x0 = (job.y - ty * I.tiles_x) * W;
     J.y0 = ty * H;
@@ -1485,7 +1613,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     // (GPUSimulators/Simulator.py:195-196, :227-228).
     if (__syncthreads_or(unhealthy) && threadIdx.x == 0) atomicOr(&ctl->bad, 1);
     if (sc.do_cfl) {
-        const float m = block_min<NT>(my_cfl, red);
+        const float m = block_min<NT>(my_cfl, red, threadIdx.x);
         if (threadIdx.x == 0) I.block_cfl[job.y] = m;
     }
     __syncthreads();
@@ -1499,7 +1627,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     float m = __int_as_float(0x7f800000);
     if (sc.do_cfl) {
         for (int i = threadIdx.x; i < I.ntiles; i += NT) m = fminf(m, __ldcg(&I.block_cfl[i]));
-        m = block_min<NT>(m, red);
+        m = block_min<NT>(m, red, threadIdx.x);
     }
     if (threadIdx.x == 0) {
         bool go = true;

@@ -116,7 +116,8 @@ FV_API int fv_sim_step(fv_sim* sim, float dt);
 /* Replaces BaseSimulator.simulate(t, dt=None) (GPUSimulators/Simulator.py:176-217):
  * advances until simTime() >= start + t.  use_dt == 0: dt = computeDt()*cfl_scale,
  * recomputed every 100 steps; use_dt != 0: the given dt.  The steps up to the next
- * recomputation run as one launch. */
+ * recomputation are one launch, or where it would take long a few; simulations of a
+ * context that run at the same time on threads of their own share the GPU. */
 FV_API int fv_sim_simulate(fv_sim* sim, double t, float dt, int use_dt);
 
 /* Advances exactly n_steps steps with the simulate() dt schedule and no end
@@ -200,7 +201,7 @@ FV_API int fv_sim_buffers(fv_sim* sim, float** ptrs, int* pitch, int* cur);
 FV_API int fv_sim_stream(fv_sim* sim, void** stream);
 
 /* Substeps per step (each a launch of its own when stepped with
- * fv_sim_substep; fv_sim_simulate runs many of them in one launch), and the
+ * fv_sim_substep; fv_sim_simulate runs many of them in a launch), and the
  * tile used (introspection for benchmarks and tests). */
 FV_API int fv_sim_info(fv_sim* sim, int* tile_w, int* tile_h, int* threads, int* launches_per_step);
 
