@@ -97,6 +97,8 @@ _SIGNATURES = {
     "fv_batch_destroy": ([_P], _I),
     "fv_batch_add": ([_P, _I, _I, _F, _F, _I, ctypes.POINTER(_FP), _I, _I, _D, ctypes.POINTER(_I)], _I),
     "fv_batch_remove": ([_P, _I], _I),
+    "fv_batch_set_shared": ([_P, _I], _I),
+    "fv_batch_launches": ([_P, ctypes.POINTER(_LL)], _I),
     "fv_batch_run": ([_P, _I], _I),
     "fv_batch_sync": ([_P], _I),
     "fv_batch_status": ([_P, _I, ctypes.POINTER(_D), ctypes.POINTER(_LL), ctypes.POINTER(_F), ctypes.POINTER(_I)],

@@ -2,8 +2,9 @@
 
 The reference runs one simulator per class instance, one kernel launch per
 substep.  A ``Batch`` holds many simulations of one scheme (any of the eight)
-resident in HBM and advances all of them with one kernel launch per run of
-several steps over a device-resident tile work list.  Each simulation
+resident in HBM and advances all of them together, over a device-resident tile
+work list: a run of several steps is one kernel launch, or where other work
+shares the GPU one per substep.  Each simulation
 follows the reference's ``simulate(t_end)`` semantics on its own: its own CFL
 time step recomputed every 100 of its steps, its last step shortened to hit
 its t_end (GPUSimulators/Simulator.py:176-217).  Its result is therefore the
@@ -29,12 +30,14 @@ def _L():
 
 
 class Batch(object):
-    """Simulations of one scheme advanced together by one batched kernel launch per run.
+    """Simulations of one scheme advanced together by a batched kernel.
     ``order`` is KP07's Runge-Kutta order (1 or 2, GPUSimulators/KP07.py:62),
-    the same for every simulation of the batch."""
+    the same for every simulation of the batch.  ``shared``: other work shares
+    the GPU with the batch, as in a server, so each substep is a launch of its
+    own; otherwise the substeps of a run are launched together."""
 
     def __init__(self, context, scheme, g=9.81, gamma=1.4, theta=None, cfl_scale=0.9, max_instances=1024,
-                 tile=None, variant=0, variant_beta=0.0, order=2):
+                 tile=None, variant=0, variant_beta=0.0, order=2, shared=False):
         if scheme not in BATCH_SCHEMES:
             raise ValueError("batched kernels exist for %s" % (BATCH_SCHEMES,))
         self.context = context
@@ -55,6 +58,7 @@ class Batch(object):
         _lib.check(_L().fv_batch_create(context.handle, _lib.SCHEME_IDS[scheme], ctypes.byref(p), int(max_instances),
                                         ctypes.byref(h)))
         self._h = h
+        _lib.check(_L().fv_batch_set_shared(h, int(bool(shared))))
         self.shapes = {}
         # slot -> (ny, nx); guarded so that a slot released by one thread and
         # taken again by another's admission keeps the new simulation's shape
@@ -95,6 +99,12 @@ class Batch(object):
     def run(self, n_steps):
         """Queue n_steps steps for every simulation (asynchronous)."""
         _lib.check(_L().fv_batch_run(self._h, int(n_steps)))
+
+    def launches(self):
+        """Stage-kernel launches of this batch so far."""
+        n = ctypes.c_longlong()
+        _lib.check(_L().fv_batch_launches(self._h, ctypes.byref(n)))
+        return n.value
 
     def sync(self):
         _lib.check(_L().fv_batch_sync(self._h))

@@ -1574,7 +1574,8 @@ int fv_host_free(void* ptr) {
 // A batch advances many simulations of one scheme together: each substep of
 // the batched kernel covers a device-resident work list of (simulation, tile)
 // pairs, every simulation keeps its own control block (t, dt, t_end, buffer
-// parity).  A run of several steps is one launch; adding or removing a
+// parity).  A run of several steps is one run of tasks, or where other work
+// shares the GPU a launch per substep (batch_in_runs); adding or removing a
 // simulation rewrites the work list between runs.
 
 struct fv_batch {
@@ -1596,7 +1597,11 @@ struct fv_batch {
     int work_buf = 0;
     int work_cap = 0;
     int nwork = 0;
-    unsigned* d_progress = nullptr;  // the launch's task counter, then the slots' progress counters
+    int largest = 0;                 // tiles of the largest simulation on the work list
+    bool shared = false;             // other work shares the GPU with this batch (fv_batch_set_shared)
+    bool counted = false;            // one of the context's running ones, from a run to the next sync
+    long long launches = 0;          // stage-kernel launches so far
+    unsigned* d_progress = nullptr;  // a run's task counter, then the slots' progress counters
     size_t progress_bytes = 0;
     int* d_err = nullptr;
     cudaStream_t copy_stream = nullptr;  // uploads/downloads, concurrent with the kernels
@@ -1630,9 +1635,33 @@ int batch_done_state(const SimCtl& c) {
     return (!(c.t < c.t_end) || cur <= 0.0f) ? 1 : 0;
 }
 
-// Queues n_steps steps of every simulation as one launch.
+void batch_uncount(fv_batch* b) {
+    std::lock_guard<std::mutex> lock(b->mu);
+    if (b->counted) b->ctx->running.fetch_sub(1, std::memory_order_relaxed);
+    b->counted = false;
+}
+
+// Whether n steps go as one run of tasks, in which the substeps of different
+// simulations overlap, or as a launch per substep.  A run holds the CTA slots
+// until its last tasks have started, so it is for a batch that has the GPU to
+// itself, and it has a progress counter to reset and to poll, which takes some
+// steps to pay.  Where one simulation has most of the tiles there is little to
+// overlap: its own substeps follow each other.  If everything is resident at
+// once that costs nothing.  us per step in runs of 16, and with a launch per
+// substep: KP07_dimsplit 20 grids of 64 to 1024 51.9, 65.8; two of 1024 50.1,
+// 55.2; one of 80 21.3, 21.4; one of 2048 89.4, 88.4; one of 1024 and eight of
+// 200 51.9, 46.9.  In runs of 4 and 1: 64 grids of 64 to 128 35.1, 36.5; 47.8,
+// 38.0.  A server with a batch per scheme served 2.70e10 cell updates per second
+// with runs of eight steps, 3.77e10 with a launch per substep.
+bool batch_in_runs(const fv_batch* b, int n_steps) {
+    if (b->shared || n_steps < 4 || b->ctx->running.load(std::memory_order_relaxed) > 1) return false;
+    return 2 * b->largest <= b->nwork || b->nwork * 6 / 5 <= b->ctx->sm_count;
+}
+
+// Queues n_steps steps of every simulation.
 int batch_launch(fv_batch* b, int n_steps) {
     fv::BatchArgs a;
+    memset(&a, 0, sizeof(a));
     a.inst = b->d_inst;
     a.ctl = b->d_ctl;
     a.work = b->d_work;
@@ -1643,10 +1672,37 @@ int batch_launch(fv_batch* b, int n_steps) {
     a.order = b->p.order;
     a.err = b->d_err;
     void* kargs[] = {&a};
-    FV_CK(cudaMemsetAsync(b->d_progress, 0, b->progress_bytes, b->stream));
-    FV_CK(cudaLaunchKernel(reinterpret_cast<const void*>(b->be->fn),
-                           dim3((unsigned)b->nwork * (unsigned)(n_steps * b->num_substeps)), dim3(b->be->NT), kargs,
-                           stage_smem(b->ctx, batch_tile_bytes(*b->be), (size_t)b->nwork), b->stream));
+    const void* fn = reinterpret_cast<const void*>(b->be->fn);
+    const dim3 block(b->be->NT);
+    const size_t tile = batch_tile_bytes(*b->be);
+    if (!batch_in_runs(b, n_steps)) {
+        a.n_sub = 1;
+        for (long long k = 0; k < (long long)n_steps * b->num_substeps; ++k) {
+            a.first_substep = (int)(k % b->num_substeps);
+            FV_CK(launch_dependent(fn, dim3((unsigned)b->nwork), block, kargs, tile, b->stream));
+            ++b->launches;
+        }
+        return FV_OK;
+    }
+    const size_t smem = stage_smem(b->ctx, tile, (size_t)b->nwork);
+    const long long per_step = (long long)b->nwork * b->num_substeps;
+    const long long chain = std::max<long long>(1, (1 << 27) / (b->be->W * b->be->H));
+    const int most = (int)std::max<long long>(1, INT_MAX / per_step);  // steps of a run
+    for (int left = n_steps; left > 0;) {
+        const int steps = std::min(left, most);
+        left -= steps;
+        a.n_sub = steps * b->num_substeps;
+        a.follows = 0;
+        FV_CK(cudaMemsetAsync(b->d_progress, 0, b->progress_bytes, b->stream));
+        for (long long tasks = per_step * steps; tasks > 0;) {
+            const unsigned ctas = (unsigned)std::min(tasks, chain);
+            tasks -= ctas;
+            a.followed = tasks > 0 ? 1 : 0;
+            FV_CK(launch_dependent(fn, dim3(ctas), block, kargs, smem, b->stream));
+            a.follows = 1;
+            ++b->launches;
+        }
+    }
     return FV_OK;
 }
 
@@ -1689,8 +1745,10 @@ int batch_publish(fv_batch* b) {
     const int k = b->work_buf ^ 1;
     FV_CK(cudaEventSynchronize(b->ev_work[k]));
     int i = 0;
+    int largest = 0;
     for (int s = 0; s < b->max_inst; ++s) {
         if (!b->used[s] || !b->registered[s]) continue;
+        largest = std::max(largest, b->h_inst[s].ntiles);
         for (int t = 0; t < b->h_inst[s].ntiles; ++t) b->h_work[k][i++] = make_int2(s, t);
     }
     if (n > 0)
@@ -1698,6 +1756,7 @@ int batch_publish(fv_batch* b) {
     FV_CK(cudaEventRecord(b->ev_work[k], b->stream));
     b->work_buf = k;
     b->nwork = n;
+    b->largest = largest;
     return FV_OK;
 }
 
@@ -1788,6 +1847,7 @@ int fv_batch_destroy(fv_batch* b) {
     if (!b) return FV_OK;
     cudaSetDevice(b->ctx->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
+    batch_uncount(b);
     for (size_t s = 0; s < b->slot_mem.size(); ++s)
         if (b->slot_mem[s]) cudaFreeAsync(b->slot_mem[s], b->stream);
     if (b->stream) cudaStreamSynchronize(b->stream);
@@ -1948,15 +2008,26 @@ int fv_batch_run(fv_batch* b, int n_steps) {
         b->dirty = false;
     }
     FV_CK(cudaEventRecord(b->ev0, b->stream));
-    if (b->nwork > 0) {
-        // One step per launch.  A launch of several holds the GPU's CTA slots until
-        // its last tiles have started, and the admissions, returns and other
-        // batches of a server wait for it: eight steps per launch served 2.70e10
-        // cell updates per second at capacity, a launch per substep 3.77e10.
-        const int most = 1;
-        for (int left = n_steps; left > 0; left -= most) FV_TRY(batch_launch(b, std::min(left, most)));
+    if (b->nwork > 0 && n_steps > 0) {
+        if (!b->counted) b->ctx->running.fetch_add(1, std::memory_order_relaxed);
+        b->counted = true;
+        FV_TRY(batch_launch(b, n_steps));
     }
     FV_CK(cudaEventRecord(b->ev1, b->stream));
+    return FV_OK;
+}
+
+int fv_batch_set_shared(fv_batch* b, int shared) {
+    if (!b) return fail(FV_ERR_INVALID, "null batch");
+    std::lock_guard<std::mutex> lock(b->mu);
+    b->shared = shared != 0;
+    return FV_OK;
+}
+
+int fv_batch_launches(fv_batch* b, long long* launches) {
+    if (!b || !launches) return fail(FV_ERR_INVALID, "bad argument");
+    std::lock_guard<std::mutex> lock(b->mu);
+    *launches = b->launches;
     return FV_OK;
 }
 
@@ -1969,7 +2040,9 @@ int fv_batch_sync(fv_batch* b) {
                               b->stream));
     }
     int err = 0;
-    FV_CK(cudaStreamSynchronize(b->stream));
+    const cudaError_t waited = cudaStreamSynchronize(b->stream);
+    batch_uncount(b);
+    FV_CK(waited);
     FV_CK(cudaMemcpy(&err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     std::lock_guard<std::mutex> lock(b->mu);
     for (int s = 0; s < b->max_inst; ++s) {

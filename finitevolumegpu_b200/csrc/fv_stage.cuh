@@ -1481,11 +1481,15 @@ struct BatchArgs {
     const BatchInstance* inst;
     SimCtl* ctl;        // control blocks, one per instance: inst[i].ctl == ctl + i
     const int2* work;   // (instance, tile within instance) per work item
-    unsigned* ticket;   // tasks taken, zero before the launch
-    unsigned* done;     // per instance, kDoneStride apart, zero before the launch: substeps of this launch
+    unsigned* ticket;   // tasks taken, zero before a run of several substeps
+    unsigned* done;     // per instance, kDoneStride apart, zero before such a run: substeps of the run
                         // completed, or kStopped once the simulation takes no further steps
     int nwork;          // work items
     int substeps;       // substeps per step
+    int first_substep;  // substep of the step that the run starts with
+    int n_sub;          // substeps of the run: of this launch, or of a chain of them
+    int follows;        // this launch goes on where the one before stopped in the same run (stage_kernel)
+    int followed;       // and the next one goes on where this one stops
     int order;          // RK order (KP07)
     int* err;           // set when a wait gave up
 };
@@ -1516,27 +1520,29 @@ __host__ __device__ constexpr int batched_blocks(int scheme, int W, int H, int N
 }
 
 // Stage kernel of any scheme over a batch: one CTA per work item and substep of
-// a launch of several steps.  Tasks are taken in order, substep by substep along
-// the work list, as in stage_kernel.  Each simulation keeps its own t, dt (its
-// own CFL every 100 of its steps) and t_end: the last of its tiles to arrive in
-// a substep updates its control block exactly as a launch of its own would, and
-// then releases the simulation's next substep.  So a substep of one simulation
-// overlaps those of the others, and the batch has no barrier.  A simulation
-// that reached its t_end, or went bad, is released for good; its tasks return.
+// a run.  A launch of one substep takes its items by block index.  The tasks of a
+// run of several steps are taken in order, substep by substep along the work
+// list, over a chain of launches if there are many, as in stage_kernel.  Each
+// simulation keeps its own t, dt (its own CFL every 100 of its steps) and t_end:
+// the last of its tiles to arrive in a substep updates its control block exactly
+// as a launch of its own would, and then releases the simulation's next substep.
+// So in a run a substep of one simulation overlaps those of the others, without a
+// barrier.  A simulation that reached its t_end, or went bad, is released for
+// good; its tasks return.
 //
-// us per step before (a launch per substep, replayed from graphs) and after:
-//                 20 grids of 64 to 1024   128 of them   1 of 2048 x 2048
-//   KP07_dimsplit          89.4   63.6      398   359        94.9  90.0
-//   HLL2                    110   81.4      508   457         119   114
-//   EE2D                    135    101      626   570         150   141
-//   KP07                   90.2   66.8      494   412         115   100
-//   WAF                     141    138      745   762         163   167
-//   HLL                    37.3   29.8      172   163        42.0  42.1
-//   FORCE                  31.3   24.9      144   137        34.9  36.5
-//   LxF                    27.5   19.4      133   115        32.2  30.9
-// (KP07's and LxF's with the registers of batched_blocks; 479, 117 and 128,
-// 32.3 before.)  A single simulation gains nothing from it: its substeps cannot
-// overlap.
+// us per step in runs of 16 steps, before (a launch per substep, replayed from
+// graphs) and now (batch_in_runs chooses a launch per substep for the last):
+//                 1 of 80 x 80  20 of 64 to 1024  128 of them  1 of 2048 x 2048
+//   KP07_dimsplit   22.3  21.3     70.3  51.9      328   288      94.8  88.4
+//   HLL2            26.1  25.3     86.1  66.0      418   363       119   110
+//   EE2D            29.2  27.8      106  81.5      514   453       149   138
+//   KP07            17.7  17.0     72.4  52.7      395   337       113  99.0
+//   WAF             21.6  20.9      116   111      599   616       162   166
+//   HLL              9.7   8.9     30.3  24.1      140   133      41.2  41.0
+//   FORCE            8.1   7.5     25.1  19.8      117   109      34.5  34.0
+//   LxF              7.9   7.3     22.7  15.3      108  93.2      32.1  28.9
+// Slower than before: WAF (its registers), and KP07 on a few grids of up to 300 x 300, 18.0 to 19.3 (its
+// bound on registers, batched_blocks).
 template <int SCHEME, int W, int H, int NT, int VAR = 0, int LPT = 1>
 __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_stage_kernel(const __grid_constant__ BatchArgs B) {
     static_assert(NT >= kInstChunks && sizeof(BatchInstance) % 16 == 0, "one thread per copied 16-byte chunk");
@@ -1547,10 +1553,17 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     __shared__ unsigned taken;
     __shared__ float red[NT / 32];
     __shared__ int flag;
-    if (threadIdx.x == 0) taken = atomicAdd(B.ticket, 1u);
-    __syncthreads();
-    const int s = (int)(taken / (unsigned)B.nwork);
-    const int2 job = B.work[taken - (unsigned)s * (unsigned)B.nwork];
+    if (!B.follows) grid_dependency_wait();  // the previous launch's states, control blocks and counters
+    unsigned item = blockIdx.x;
+    int s = 0;
+    if (B.n_sub > 1) {
+        if (threadIdx.x == 0) taken = atomicAdd(B.ticket, 1u);
+        __syncthreads();
+        s = (int)(taken / (unsigned)B.nwork);
+        item = taken - (unsigned)s * (unsigned)B.nwork;
+        if (B.followed) grid_launch_dependents();
+    }
+    const int2 job = B.work[item];
     prefetch_instance(&I, B.inst + job.x);
     unsigned* const done = B.done + (size_t)kDoneStride * job.x;
     SimCtl* const ctl = B.ctl + job.x;
@@ -1576,12 +1589,16 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     }
     cp_async_wait_all();
     __syncthreads();
-    if (flag) return;
-    const int sub = s % B.substeps;
+    if (flag) {
+        if (B.follows) grid_dependency_wait();
+        return;
+    }
+    const int sub = (B.first_substep + s) % B.substeps;
     const bool is_last = sub == B.substeps - 1;  // of its step
     StepCtl sc = step_from_words(words[0], words[1], words[2], false, 0.0f, false, is_last);
     if (!sc.active) {  // from the launch's start: later it is released as stopped
-        if (job.y == 0 && threadIdx.x == 0) st_release(done, kStopped);
+        if (B.n_sub > 1 && job.y == 0 && threadIdx.x == 0) st_release(done, kStopped);
+        if (B.follows) grid_dependency_wait();
         return;
     }
     if (SCHEME == WAF) sc.do_cfl = false;  // WAFKernel has no CFL output (SWE2D_WAF.cu:103-119)
@@ -1610,7 +1627,9 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
     }
     // The tile's CFL minimum, its arrival, and in the last tile of the
     // simulation to arrive the control-block update of Simulator.step / simulate
-    // (GPUSimulators/Simulator.py:195-196, :227-228).
+    // (GPUSimulators/Simulator.py:195-196, :227-228).  The tile is written: the
+    // next launch's CTAs may start, and wait for the end of this one.
+    if (!B.followed) grid_launch_dependents();
     if (__syncthreads_or(unhealthy) && threadIdx.x == 0) atomicOr(&ctl->bad, 1);
     if (sc.do_cfl) {
         const float m = block_min<NT>(my_cfl, red, threadIdx.x);
@@ -1622,6 +1641,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
         flag = atomicAdd(&ctl->arrive, 1u) == (unsigned)I.ntiles - 1u;
     }
     __syncthreads();
+    if (B.follows) grid_dependency_wait();
     if (!flag) return;
     __threadfence();
     float m = __int_as_float(0x7f800000);
@@ -1642,7 +1662,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
             go = ctl->t < ctl->t_end && !((float)((rem < d) ? rem : d) <= 0.0f);  // step_from_words
         }
         ctl->arrive = 0u;
-        st_release(done, go ? (unsigned)s + 1u : kStopped);
+        if (B.n_sub > 1) st_release(done, go ? (unsigned)s + 1u : kStopped);
     }
 }
 

@@ -128,7 +128,7 @@ class Server(object):
         if b is None:
             scheme, g, gamma = key
             b = self.batches[key] = Batch(self.context, scheme, g=g, gamma=gamma, cfl_scale=self.cfl_scale,
-                                          max_instances=self.max_instances)
+                                          max_instances=self.max_instances, shared=True)
         return b
 
     def serve(self, requests: List[Request], clock=time.perf_counter, result_fn=None):

@@ -229,13 +229,21 @@ FV_API int fv_batch_destroy(fv_batch* batch);
 FV_API int fv_batch_add(fv_batch* batch, int nx, int ny, float dx, float dy, int bc, const float* const* host_vars,
                         int host_rows, int host_cols, double t_end, int* slot);
 FV_API int fv_batch_remove(fv_batch* batch, int slot);
-/* Queues n_steps steps for every simulation of the batch (one launch of the
- * batched kernel, over all substeps and the tile work list);
+/* Queues n_steps steps for every simulation of the batch, as one launch over all
+ * of them or as a launch per substep (fv_batch_set_shared);
  * simulations that reached t_end do nothing. Asynchronous.
  * Simulations admitted or removed since the last run join or leave the tile
  * work list first; FV_ERR_NOMEM means the list could not grow, nothing was
  * queued and the batch is unchanged (a later call retries). */
 FV_API int fv_batch_run(fv_batch* batch, int n_steps);
+/* shared != 0: other work shares the GPU with this batch (other batches, admissions
+ * between short runs), so each substep is a launch of its own and the others' work
+ * gets its turn between them.  0 (the default): where nothing else of the context
+ * runs, the substeps of a run are one launch, or a few, in which those of different
+ * simulations overlap. */
+FV_API int fv_batch_set_shared(fv_batch* batch, int shared);
+/* Stage-kernel launches of this batch so far. */
+FV_API int fv_batch_launches(fv_batch* batch, long long* launches);
 /* Waits for queued work and refreshes the host view of every simulation. */
 FV_API int fv_batch_sync(fv_batch* batch);
 /* t, nt, dt and the simulation's state as of the last sync: done = 0 still
