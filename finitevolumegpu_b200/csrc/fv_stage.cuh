@@ -317,7 +317,7 @@ __device__ __forceinline__ float sign_y(int v) { return v == 2 ? -1.0f : 1.0f; }
 // wrapped cell from global memory, then reflective sides mirror interior cells
 // with the normal momentum negated, north, south, east, west in turn.
 // Dirichlet ghosts keep the stored values the TMA load brought in.
-template <int NV, int W, int H, int NT, int SP, bool LOOP>
+template <int NV, int W, int H, int NT, int SP, bool LOOP, int UNROLL>
 __device__ void apply_boundary(float* Qs, const TileJob& J) {
     constexpr int TR = H + 4, PS = SP * TR;
     const int nx = J.nx, ny = J.ny, bc = J.bc, x0 = J.x0, y0 = J.y0;
@@ -332,12 +332,13 @@ __device__ void apply_boundary(float* Qs, const TileJob& J) {
         // Periodic walls, us per step before and after (reflective walls):
         // KP07_dimsplit 256 x 256 13.8, 10.6 (9.9), 777 x 1333 with 60 x 60
         // tiles 40.3, 28.1 (23.2); EE2D 2048 x 2048 113, 108 (104); FORCE
-        // 777 x 1333 11.9, 8.9 (7.9).
+        // 777 x 1333 11.9, 8.9 (7.9).  UNROLL: loads of a variable in flight per
+        // thread (batched_blocks has the reason for fewer).
         const int row_n = ny - y0 + 2, col_e = nx - x0 + 4;  // tile row of y = ny, tile column of x = nx
         const int lo_r = (ps && y0 == 0) ? 2 : 0, hi_r = pn ? max(0, min(2, TR - row_n)) : 0;
         const int lo_c = (pw && x0 == 0) ? 2 : 0, hi_c = pe ? max(0, min(2, SP - col_e)) : 0;
         const int in_rows = (lo_r + hi_r) * SP, all = in_rows + (lo_c + hi_c) * TR;
-#pragma unroll 4
+#pragma unroll UNROLL
         for (int i = thread_of<LOOP>(J.tid); i < all; i += NT) {
             int t, s;
             bool use = true;
@@ -851,7 +852,7 @@ __device__ bool process_tile_dimsplit(float* Qs, uint64_t* bar, uint32_t phase, 
         if (!load_tile<NV, SP, TR, LOOP>(Qs, J.tmap, J.x0, J.y0, bar, phase, init_bar, J.tid, err, polls)) return false;
     }
     const int x0 = J.x0, y0 = J.y0;
-    if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<NV, W, H, NT, SP, LOOP>(Qs, J);
+    if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<NV, W, H, NT, SP, LOOP, (SCHEME == WAF && ASYNC_LOAD) ? 1 : 4>(Qs, J);
 
     SweepPar p;
     p.theta = P.theta;
@@ -1012,7 +1013,7 @@ __device__ bool process_tile_unsplit(float* Qs, uint64_t* bar, uint32_t phase, b
         if (!load_tile<3, SP, TR, LOOP>(Qs, J.tmap, x0, y0, bar, phase, init_bar, thread_of<LOOP>(J.tid), err, polls)) return false;
     }
     {
-        if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<3, W, H, NT, SP, LOOP>(Qs, J);
+        if (x0 == 0 || x0 + W + 2 > J.nx || y0 == 0 || y0 + H + 2 > J.ny) apply_boundary<3, W, H, NT, SP, LOOP, 4>(Qs, J);
         const float kdt = P.kdt;
         const float g = P.g, half_g = fmul(0.5f, g), theta2 = minmod_theta2(P.theta);
         const float k4x = fdiv_fast(P.dx, fmul(4.0f, kdt)), k4y = fdiv_fast(P.dy, fmul(4.0f, kdt));
@@ -1510,9 +1511,13 @@ __device__ __forceinline__ void prefetch_instance(BatchInstance* m, const BatchI
 // take 64 and 80.  us per step, 128 grids of 64 to 1024 cells a side and one of
 // 2048: LxF 139 to 115 and 34.6 to 30.6, KP07 513 to 408 and 123 to 99.7 (eight:
 // 388 and 103, but spilling, and 64 grids of 64 to 128 take 27.6 instead of
-// 23.9; six: 24.9).  WAF with six: 761 to 740, but 64 small grids 47.8 to 54.3.
+// 23.9; six: 24.9).  WAF's 28-row tiles would take 101, which is one CTA less than
+// five: bound to five 622 to 610 and 166 to 163, and with the periodic ghost
+// cells' loads one after the other 594 and 160 (six CTAs: 64 small grids 47.8 to
+// 54.3).
 __host__ __device__ constexpr int batched_blocks(int scheme, int W, int H, int NT) {
     const int most = 65536 / (NT * 128);
+    if (scheme == WAF && H == 28 && NT == 128) return 5;
     if (scheme != LXF && scheme != KP07) return most;
     const int by_smem = 228 * 1024 / (3 * (W + 8) * (H + 4) * (int)sizeof(float) + 1024 + 256);  // 228 KB per SM
     const int wanted = scheme == LXF ? 8 : 6;
@@ -1537,11 +1542,11 @@ __host__ __device__ constexpr int batched_blocks(int scheme, int W, int H, int N
 //   HLL2            26.1  25.3     86.1  66.0      418   363       119   110
 //   EE2D            29.2  27.8      106  81.5      514   453       149   138
 //   KP07            17.7  17.0     72.4  52.7      395   337       113  99.0
-//   WAF             21.6  20.9      116   111      599   616       162   166
+//   WAF             21.6  21.1      116   106      599   589       162   160
 //   HLL              9.7   8.9     30.3  24.1      140   133      41.2  41.0
 //   FORCE            8.1   7.5     25.1  19.8      117   109      34.5  34.0
 //   LxF              7.9   7.3     22.7  15.3      108  93.2      32.1  28.9
-// Slower than before: WAF (its registers), and KP07 on a few grids of up to 300 x 300, 18.0 to 19.3 (its
+// Slower than before: KP07 on a few grids of up to 300 x 300, 18.0 to 19.3 (its
 // bound on registers, batched_blocks).
 template <int SCHEME, int W, int H, int NT, int VAR = 0, int LPT = 1>
 __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_stage_kernel(const __grid_constant__ BatchArgs B) {
