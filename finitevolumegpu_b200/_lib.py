@@ -108,6 +108,8 @@ _SIGNATURES = {
                        ctypes.POINTER(_D)], _I),
     "fv_batch_tile": ([_P, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I)], _I),
     "fv_sim_set_wait_limit": ([_P, _I], _I),
+    "fv_sim_set_neighbour_wait_limit": ([_P, _I], _I),
+    "fv_batch_set_wait_limit": ([_P, _I], _I),
     "fv_selftest_bounded_wait": ([_I, ctypes.POINTER(_I)], _I),
     "fv_host_alloc": ([ctypes.POINTER(_P), ctypes.c_size_t], _I),
     "fv_host_free": ([_P], _I),

@@ -780,7 +780,11 @@ int read_ctl(fv_sim* s) {
         FV_CK(cudaStreamSynchronize(s->stream));
         s->ctl_known = true;
     }
-    if (s->ctl_h->error) return fail(FV_ERR_DEVICE, "a stage kernel gave up waiting for its tile load");
+    if (s->ctl_h->error)
+        return fail(FV_ERR_DEVICE, "a stage kernel gave up waiting for %s",
+                    s->ctl_h->error == fv::kTileLoadGaveUp    ? "its tile load"
+                    : s->ctl_h->error == fv::kNeighbourGaveUp ? "a neighbouring tile"
+                                                              : "its tile load, another one for a neighbouring tile");
     return FV_OK;
 }
 
@@ -1475,10 +1479,20 @@ int fv_sim_set_boundary_conditions(fv_sim* s, int bc) {
     return FV_OK;
 }
 
+// A limit in polls (negative: the default) as the kernels' arguments have it.
+static int wait_limit(int polls) { return polls < 0 ? 0 : (polls == 0 ? -1 : polls); }
+
 int fv_sim_set_wait_limit(fv_sim* s, int polls) {
     FV_TRY(check_sim(s));
     FV_CK(cudaStreamSynchronize(s->stream));
-    s->args.wait_limit = polls < 0 ? 0 : (polls == 0 ? -1 : polls);
+    s->args.wait_limit = s->args.neighbour_limit = wait_limit(polls);
+    return FV_OK;
+}
+
+int fv_sim_set_neighbour_wait_limit(fv_sim* s, int polls) {
+    FV_TRY(check_sim(s));
+    FV_CK(cudaStreamSynchronize(s->stream));
+    s->args.neighbour_limit = wait_limit(polls);
     return FV_OK;
 }
 
@@ -1601,6 +1615,7 @@ struct fv_batch {
     bool shared = false;             // other work shares the GPU with this batch (fv_batch_set_shared)
     bool counted = false;            // one of the context's running ones, from a run to the next sync
     long long launches = 0;          // stage-kernel launches so far
+    int wait_limit = 0;              // of the kernels' waits (BatchArgs)
     unsigned* d_progress = nullptr;  // a run's task counter, then the slots' progress counters
     size_t progress_bytes = 0;
     int* d_err = nullptr;
@@ -1671,6 +1686,7 @@ int batch_launch(fv_batch* b, int n_steps) {
     a.substeps = b->num_substeps;
     a.order = b->p.order;
     a.err = b->d_err;
+    a.wait_limit = b->wait_limit;
     void* kargs[] = {&a};
     const void* fn = reinterpret_cast<const void*>(b->be->fn);
     const dim3 block(b->be->NT);
@@ -2024,6 +2040,13 @@ int fv_batch_set_shared(fv_batch* b, int shared) {
     return FV_OK;
 }
 
+int fv_batch_set_wait_limit(fv_batch* b, int polls) {
+    if (!b) return fail(FV_ERR_INVALID, "null batch");
+    std::lock_guard<std::mutex> lock(b->mu);
+    b->wait_limit = wait_limit(polls);
+    return FV_OK;
+}
+
 int fv_batch_launches(fv_batch* b, long long* launches) {
     if (!b || !launches) return fail(FV_ERR_INVALID, "bad argument");
     std::lock_guard<std::mutex> lock(b->mu);
@@ -2052,7 +2075,7 @@ int fv_batch_sync(fv_batch* b) {
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, b->ev0, b->ev1) == cudaSuccess) b->last_ms = ms;
     cudaGetLastError();
-    if (err) return fail(FV_ERR_DEVICE, "a batched stage kernel gave up waiting for a tile load");
+    if (err) return fail(FV_ERR_DEVICE, "a batched stage kernel gave up waiting for an earlier substep of its simulation");
     return FV_OK;
 }
 

@@ -45,6 +45,10 @@ __host__ __device__ inline int bc_south(int bc) { return (bc >> 16) & 0xF; }
 __host__ __device__ inline int bc_east(int bc) { return (bc >> 8) & 0xF; }
 __host__ __device__ inline int bc_west(int bc) { return bc & 0xF; }
 
+// What a bounded wait that gave up was for.
+constexpr int kTileLoadGaveUp = 1;   // the tensor copies of a tile
+constexpr int kNeighbourGaveUp = 2;  // the tiles around it in the substep before
+
 // Control block of one simulation, resident in device memory.
 struct alignas(16) SimCtl {
     double t;          // simulation time (BaseSimulator.t, FP64)
@@ -57,7 +61,7 @@ struct alignas(16) SimCtl {
     int update_dt;     // recompute dt every 100 steps (simulate(t) without dt)
     int cur;           // buffer index holding u0
     unsigned int arrive;  // CTA arrival counter for the last-CTA epilogue
-    int error;         // nonzero once a bounded wait gave up
+    int error;         // kTileLoadGaveUp, kNeighbourGaveUp: the bounded waits that gave up
     int bad;           // batched simulations: a step left a non-finite value or a non-positive depth
                        // (density); the simulation then stops (t_end is set to t)
 };
@@ -96,8 +100,9 @@ struct StageArgs {
     int explicit_dt;     // all steps take dt_step, whatever the control block says
     float dt_step;
     int want_cfl;        // compute the CFL minimum of the last substep's state
-    int wait_limit;      // bounded waits: 0 = kWaitPolls polls (the default, also for zero-filled
-                         // arguments), n > 0 = n polls, negative = give up at once (tests)
+    int wait_limit;      // bounded waits for tile loads: 0 = kWaitPolls polls (the default, also for
+                         // zero-filled arguments), n > 0 = n polls, negative = give up at once (tests)
+    int neighbour_limit; // the same for the waits for neighbouring tiles
     int follows;         // this launch goes on where the one before stopped in the same run of substeps
     int followed;        // and the next one goes on where this one stops
     int tile_row0;       // first tile row of this launch (one substep may be split into launches by rows)
@@ -267,7 +272,7 @@ __device__ __forceinline__ bool load_tile(float* Qs, const CUtensorMap* tmap, in
     const bool ok = mbar_wait_bounded(bar, phase, polls);
     const int failed = __syncthreads_or(ok ? 0 : 1);
     if (failed) {
-        if (thread_of<LOOP>(tid) == 0) atomicExch(err, 1);
+        if (thread_of<LOOP>(tid) == 0) atomicOr(err, kTileLoadGaveUp);
         mbar_wait_bounded(bar, phase, kWaitPolls);  // let copies in flight land before the CTA moves on
         return false;
     }
@@ -1321,7 +1326,7 @@ __global__ void __launch_bounds__(NT, compiled_blocks(SCHEME, W, H, NT, LPT)) st
             const int ny = near_tile(ty, j, A.ny, A.tiles_y, H, wrap_y);
             if (tid == 15 || nx != tx || ny != ty) {  // thread 15 waits for the tile itself
                 const unsigned* p = A.done + (size_t)kDoneStride * (ny * A.tiles_x + nx);
-                const uint32_t polls = wait_polls(A.wait_limit);
+                const uint32_t polls = wait_polls(A.neighbour_limit);
                 ok = false;
                 for (uint32_t k = 0; k < polls; ++k) {
                     if (ld_acquire(p) >= (unsigned)s) {
@@ -1374,8 +1379,8 @@ __global__ void __launch_bounds__(NT, compiled_blocks(SCHEME, W, H, NT, LPT)) st
                 broken = !loaded;  // its barrier's phase is not known any more: no further load
             }
             fence_proxy_async_global();  // these stores precede other tiles' tensor copies
-        } else if (!run && tid == 0) {
-            atomicExch(&A.ctl->error, 1);
+        } else if (!run && tid == 0 && !(LOOP && broken)) {
+            atomicOr(&A.ctl->error, kNeighbourGaveUp);
         }
         const int tile = ty * A.tiles_x + tx;
         if constexpr (LOOP) {  // (below for the others)
@@ -1493,6 +1498,7 @@ struct BatchArgs {
     int followed;       // and the next one goes on where this one stops
     int order;          // RK order (KP07)
     int* err;           // set when a wait gave up
+    int wait_limit;     // polls of the bounded waits, as StageArgs' (0: the default)
 };
 constexpr unsigned kStopped = 0xffffffffu;
 
@@ -1576,7 +1582,7 @@ __global__ void __launch_bounds__(NT, batched_blocks(SCHEME, W, H, NT)) batched_
         unsigned seen = 0u;
         if (s > 0) {
             // bounded; one wait that gives up ends all of them
-            for (uint32_t k = 0; k < kWaitPolls; ++k) {
+            for (uint32_t k = 0; k < wait_polls(B.wait_limit); ++k) {
                 seen = ld_acquire(done);
                 if (seen >= (unsigned)s || *(volatile int*)B.err) break;
                 __nanosleep(20);

@@ -166,12 +166,16 @@ FV_API int fv_sim_set_boundary_conditions(fv_sim* sim, int bc);
 /* Test hooks (no counterpart in the reference): the give-up path of the
  * stage kernels' bounded waits, exercised without faulting or hanging a GPU.
  * fv_sim_set_wait_limit sets how many times a stage kernel polls for its
- * tile load before it gives up (negative: the default, about a second); 0
- * gives up at once, after which the kernel still waits, boundedly, for its
- * copies to land, writes nothing and the next synchronising call returns
- * FV_ERR_DEVICE.  fv_selftest_bounded_wait runs one warp that waits `polls`
+ * tile load, and for the tiles around it in the substep before, until it gives
+ * up (negative: the default, about a second); 0 gives up at once, after which
+ * the kernel still waits, boundedly, for its copies to land, writes nothing and
+ * the next synchronising call returns FV_ERR_DEVICE and says which wait it was.
+ * fv_sim_set_neighbour_wait_limit sets the limit of the second wait alone,
+ * fv_batch_set_wait_limit that of a batch's wait for its simulations' earlier
+ * substeps, for the runs that follow.  fv_selftest_bounded_wait runs one warp that waits `polls`
  * times on a barrier that nothing completes; *gave_up = 1 when it gave up. */
 FV_API int fv_sim_set_wait_limit(fv_sim* sim, int polls);
+FV_API int fv_sim_set_neighbour_wait_limit(fv_sim* sim, int polls);
 FV_API int fv_selftest_bounded_wait(int polls, int* gave_up);
 
 /* Time-stepping state of a simulation: simulated time t, steps nt, the
@@ -242,6 +246,7 @@ FV_API int fv_batch_run(fv_batch* batch, int n_steps);
  * runs, the substeps of a run are one launch, or a few, in which those of different
  * simulations overlap. */
 FV_API int fv_batch_set_shared(fv_batch* batch, int shared);
+FV_API int fv_batch_set_wait_limit(fv_batch* batch, int polls);
 /* Stage-kernel launches of this batch so far. */
 FV_API int fv_batch_launches(fv_batch* batch, long long* launches);
 /* Waits for queued work and refreshes the host view of every simulation. */
