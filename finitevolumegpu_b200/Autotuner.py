@@ -41,10 +41,9 @@ TILE_CONFIGS = {
     "LxF": 6,
     "KP07": 6,
 }
-# KP07_dimsplit's 12 x 12 tile (configuration 11) is a candidate below this many
-# cells only: from 256 x 256 on, the tiles reported for the scheme stay those of
-# 28, 60 and 124 columns.
-SMALL_TILE_CELLS = {"KP07_dimsplit": (11, 256 * 256)}
+# The 12 x 12 tiles, for grids that do not fill the GPU: get_peak_performance()
+# reports the tiles of 28 columns and more, as its callers know them.
+SMALL_TILES = {"KP07_dimsplit": 11, "HLL2": 11, "WAF": 11, "EE2D_KP07_dimsplit": 10, "FORCE": 4, "HLL": 4}
 # Tile configurations of the batched kernels per scheme.
 BATCH_TILE_CONFIGS = {
     "LxF": 2,
@@ -161,8 +160,7 @@ class Autotuner(object):
                 del sim
             finally:
                 context.autotuner = ctx_tuner
-        small, cells = SMALL_TILE_CELLS.get(scheme, (None, 0))
-        best = min((k for k in results if k != small or nx * ny < cells), key=results.get)
+        best = min(results, key=results.get)
         cache = self._load()
         cache.setdefault(context.device_name, {}).setdefault(scheme, {})[size_class(nx, ny)] = {
             "tile": best,
@@ -198,9 +196,10 @@ class Autotuner(object):
         self.performance.pop(key, None)
 
     def get_peak_performance(self, simulator):
-        """{"block_width", "block_height", "megacells"} of the fastest tile for
-        `simulator` at nx x ny, benchmarking first if needed
-        (GPUSimulators/Autotuner.py:104-146)."""
+        """{"block_width", "block_height", "megacells"} of the fastest tile of 28
+        columns or more for `simulator` at nx x ny, benchmarking first if needed
+        (GPUSimulators/Autotuner.py:104-146).  Simulators take the fastest of all
+        (get_tile)."""
         key = simulator.__name__
         if key in self.performance:
             return self.performance[key]
@@ -212,7 +211,10 @@ class Autotuner(object):
         from . import SCHEMES
 
         cls = SCHEMES[key]
-        tuner, ctx.autotuner = ctx.autotuner, _Fixed(int(entry["tile"]))
+        tile, ms = int(entry["tile"]), float(entry["ms_per_step"])
+        if tile == SMALL_TILES.get(key):
+            ms, tile = min((float(v), int(k)) for k, v in entry["all"].items() if int(k) != tile)
+        tuner, ctx.autotuner = ctx.autotuner, _Fixed(tile)
         try:  # the tile's shape, from a small simulator built with it
             q = [np.ones((8, 8), np.float32), np.zeros((8, 8), np.float32), np.zeros((8, 8), np.float32)]
             if key == "EE2D_KP07_dimsplit":
@@ -224,7 +226,7 @@ class Autotuner(object):
         finally:
             ctx.autotuner = tuner
         self.performance[key] = {"block_width": info["tile_w"], "block_height": info["tile_h"],
-                                 "megacells": self.nx * self.ny / (float(entry["ms_per_step"]) * 1e-3) / 1e6}
+                                 "megacells": self.nx * self.ny / (ms * 1e-3) / 1e6}
         return self.performance[key]
 
     @staticmethod
