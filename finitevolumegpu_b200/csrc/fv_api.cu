@@ -1820,8 +1820,12 @@ int fv_batch_create(fv_context* ctx, int scheme, const fv_params* params, int ma
         fv_batch_destroy(b);
         return rc;
     };
-    // Uploads zero their memory and estimate the first dt with kernels: a higher
-    // priority starts them ahead of the tiles that a batched launch still queues.
+    // The zeroing of an admitted simulation's memory and the copies of uploads and
+    // downloads, ahead of the tiles that a batched launch still queues.  (The first
+    // dt estimate of an admission runs on the batch's own stream: kernels queued
+    // there may still use the slot's control block.)  4000 requests at 1200 per
+    // second, six runs each: 3.5e10 to 4.1e10 cell updates per second, at normal
+    // priority 2.7e10 to 4.0e10.
     int lowest = 0, copy_priority = 0;
     cudaDeviceGetStreamPriorityRange(&lowest, &copy_priority);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
