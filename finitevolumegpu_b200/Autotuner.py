@@ -48,7 +48,7 @@ SMALL_TILES = {"KP07_dimsplit": 11, "HLL2": 11, "WAF": 11, "EE2D_KP07_dimsplit":
 BATCH_TILE_CONFIGS = {
     "LxF": 2,
     "KP07": 2,
-    "KP07_dimsplit": 7,
+    "KP07_dimsplit": 5,
     "HLL": 4,
     "EE2D_KP07_dimsplit": 4,
     "HLL2": 4,

@@ -249,9 +249,6 @@ const BEntry kBatchTable[] = {
     {FV_HLL2, 60, 60, 128, batch_fn<fv::HLL2, 60, 60, 128, 0, 2>()},
     {FV_WAF, 60, 60, 128, batch_fn<fv::WAF, 60, 60, 128, 0, 2>()},
     {FV_EE2D_KP07_DIMSPLIT, 60, 60, 128, batch_fn<fv::EE2D, 60, 60, 128, 0, 2>()},
-    // (tile indices that tuner caches may hold)
-    {FV_KP07_DIMSPLIT, 60, 60, 128, batch_fn<fv::KP07_DIMSPLIT, 60, 60, 128, 0, 2>()},
-    {FV_KP07_DIMSPLIT, 124, 28, 128, batch_fn<fv::KP07_DIMSPLIT, 124, 28, 128>()},
 };
 constexpr int kNumBatchEntries = sizeof(kBatchTable) / sizeof(kBatchTable[0]);
 
@@ -335,6 +332,8 @@ const BEntry* find_batch_entry(int scheme, int cfg, int variant) {
                 return &kBatchVariantTable[i].b;
         return nullptr;
     }
+    // the indices of two forms of tiles 4 and 1 that are gone, which caches may hold
+    if (scheme == FV_KP07_DIMSPLIT && (cfg == 5 || cfg == 6)) cfg = cfg == 5 ? 4 : 1;
     int k = 0;
     for (int i = 0; i < kNumBatchEntries; ++i) {
         if (kBatchTable[i].scheme != scheme) continue;

@@ -116,3 +116,10 @@ def test_run_in_a_chain_of_launches(ctx):
             assert b.status(k)["nt"] == s.simSteps()
             for x, y in zip(b.download(k), s.download()):
                 assert np.array_equal(x, y)
+
+
+def test_retired_tile_indices_are_accepted(ctx):
+    """Indices 5 and 6 of KP07_dimsplit, which older timing caches may hold."""
+    for old, now in ((5, 4), (6, 1)):
+        a, b = (Batch(ctx, "KP07_dimsplit", tile=t, max_instances=2).info() for t in (old, now))
+        assert [a[k] for k in ("tile_w", "tile_h", "threads")] == [b[k] for k in ("tile_w", "tile_h", "threads")]

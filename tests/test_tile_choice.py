@@ -45,3 +45,16 @@ def test_benchmark_records_the_fastest_and_peak_reports_the_widest_known(tmp_pat
     assert Autotuner(cache_file=str(tmp_path / "cache.json")).get_tile("KP07_dimsplit", 256, 256, "Dev") == 11
     assert peak["block_width"] == 28 and np.isclose(peak["megacells"], 256 * 256 / 0.75e-3 / 1e6)
     assert set(module.SMALL_TILES) <= set(module.TILE_CONFIGS)
+
+
+def test_no_batched_kernel_is_listed_twice():
+    """The tuner times every row of the batched kernels' table."""
+    import os
+    import re
+
+    from conftest import ROOT
+
+    src = open(os.path.join(ROOT, "finitevolumegpu_b200", "csrc", "fv_api.cu")).read()
+    rows = re.findall(r"batch_fn<([^>]*)>\(\)", re.search(r"BEntry kBatchTable\[\] = \{(.*?)\n\};", src, re.S).group(1))
+    rows = [tuple((r.replace(" ", "").split(",") + ["0", "1"])[:6]) for r in rows]
+    assert len(rows) > 20 and len(set(rows)) == len(rows)
