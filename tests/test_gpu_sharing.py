@@ -158,3 +158,24 @@ def test_small_simulation_beside_a_large_one(ctx):
 
     side_by_side([run_big, run_small])
     assert sorted(waits)[5] < 0.3 * alone, (waits, alone)
+
+
+def test_steps_on_threads_equal_steps_alone(ctx):
+    """step() with and without another simulation in the context."""
+    nx, ny = 300, 310
+    alone = make(ctx, "KP07_dimsplit", nx, ny)
+    dt = np.float32(alone.computeDt() * np.float32(0.4))
+
+    def run(s):
+        for _ in range(40):
+            s.step(dt)
+        s.synchronize()
+
+    run(alone)
+    want = alone.download()
+    sims = [make(ctx, "KP07_dimsplit", nx, ny) for _ in range(4)]
+    side_by_side([lambda s=s: run(s) for s in sims])
+    for s in sims:
+        assert s.simSteps() == 40 and s.computeDt() == alone.computeDt()
+        for x, y in zip(s.download(), want):
+            assert np.array_equal(x, y)
