@@ -592,7 +592,7 @@ struct fv_context {
     HostStaging staging;
     CtlSlab ctl_slab;
     std::atomic<int> running{0};  // simulations in simulate() or advance(), batches between a run and a sync
-    std::atomic<int> sims{0};     // simulations that exist
+    std::atomic<int> members{0};  // simulations and batches that exist
 };
 
 // A simulation's looping kernel with one of its tiles.
@@ -934,12 +934,18 @@ int loop_form(fv_sim* s, const LoopForm** form, unsigned* ctas) {
     return FV_OK;
 }
 
-// Tasks of a launch of a chain: 2^27 cell updates, a millisecond or less, which
-// is what other streams wait for at most.  20 steps of a 256 x 256 grid beside a
-// 4096 x 4096 one: 3.2 ms with a launch per substep, 25.5 in launches of 100
-// steps, 1.1 in chains; 0.5 in chains of an eighth of the size, which cost LxF
-// 3 % on 4096 x 4096.
-long long chain_tasks(const fv_sim* s) { return (1 << 27) / (s->ke->W * s->ke->H); }
+// Cell updates of a launch of a chain, which is what other streams wait for at
+// most: 2^24, a tenth of a millisecond, where the context has other simulations
+// or batches, which may run at any time, and 2^26 where it has none.  256 x 256
+// steps beside a 4096 x 4096 run, ms, with a launch per substep, launches of 100
+// steps, and chains of 2^27, 2^26, 2^24 and 2^22: one step 0.15, 13.4, 0.97, 0.52,
+// 0.13, 0.06; two 0.46, 23.8, 1.0, 0.53, 0.15, 0.09; twenty 3.2, 25.5, 2.8, 2.3,
+// 2.1, 2.3.  us per step on 4096 x 4096 in one launch and in the same chains:
+// KP07_dimsplit 260.8, 261.3, 261.6, 261.6, 263.3; LxF 84.4, 84.4, 84.8, 86.9, 95.7.
+int chain_cells(const fv_context* ctx) {
+    return ctx->members.load(std::memory_order_relaxed) > 1 ? 1 << 24 : 1 << 26;
+}
+long long chain_tasks(const fv_sim* s) { return chain_cells(s->ctx) / (s->ke->W * s->ke->H); }
 
 // Steps of a run in the looping form: 2^24 cell updates, after which a run takes
 // the share of the then current number of simulations (a quarter of them loses
@@ -975,10 +981,10 @@ int launch_stage(fv_sim* s, const StagePlan& p) {
         ++s->launches;
     } else {
         const long long most = p.n_sub > 1 ? chain_tasks(s) : tiles;
-        // step()'s few substeps: padded where there is no other simulation whose
-        // steps could run beside them (1024 x 1024 alone 35.7 us instead of 39.0;
+        // step()'s few substeps: padded where there is nothing else that could run
+        // beside them (1024 x 1024 alone 35.7 us instead of 39.0;
         // on 8 threads 22.0 instead of 20.9, 256 x 256 8.2 instead of 6.6)
-        const bool padded = p.n_sub > s->num_substeps || (p.n_sub > 1 && s->ctx->sims.load(std::memory_order_relaxed) == 1);
+        const bool padded = p.n_sub > s->num_substeps || (p.n_sub > 1 && s->ctx->members.load(std::memory_order_relaxed) == 1);
         for (long long left = (long long)tiles * p.n_sub; left > 0;) {
             const unsigned ctas = (unsigned)std::min(left, most);
             left -= ctas;
@@ -1115,7 +1121,7 @@ int fv_sim_create(fv_context* ctx, int scheme, int nx, int ny, float dx, float d
 
     fv_sim* s = new fv_sim;
     s->ctx = ctx;
-    ctx->sims.fetch_add(1, std::memory_order_relaxed);
+    ctx->members.fetch_add(1, std::memory_order_relaxed);
     s->scheme = scheme;
     s->nx = nx;
     s->ny = ny;
@@ -1247,7 +1253,7 @@ int fv_sim_destroy(fv_sim* s) {
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->stream) cudaStreamDestroy(s->stream);
-    s->ctx->sims.fetch_sub(1, std::memory_order_relaxed);
+    s->ctx->members.fetch_sub(1, std::memory_order_relaxed);
     delete s;
     return FV_OK;
 }
@@ -1708,7 +1714,7 @@ int batch_launch(fv_batch* b, int n_steps) {
     }
     const size_t smem = stage_smem(b->ctx, tile, (size_t)b->nwork);
     const long long per_step = (long long)b->nwork * b->num_substeps;
-    const long long chain = std::max<long long>(1, (1 << 27) / (b->be->W * b->be->H));
+    const long long chain = chain_cells(b->ctx) / (b->be->W * b->be->H);
     const int most = (int)std::max<long long>(1, INT_MAX / per_step);  // steps of a run
     for (int left = n_steps; left > 0;) {
         const int steps = std::min(left, most);
@@ -1807,6 +1813,7 @@ int fv_batch_create(fv_context* ctx, int scheme, const fv_params* params, int ma
                                100));
     fv_batch* b = new fv_batch;
     b->ctx = ctx;
+    ctx->members.fetch_add(1, std::memory_order_relaxed);
     b->scheme = scheme;
     b->nv = scheme_nv(scheme);
     b->gc = scheme_ghost(scheme);
@@ -1898,6 +1905,7 @@ int fv_batch_destroy(fv_batch* b) {
         cudaStreamDestroy(b->copy_stream);
     }
     if (b->stream) cudaStreamDestroy(b->stream);
+    b->ctx->members.fetch_sub(1, std::memory_order_relaxed);
     delete b;
     return FV_OK;
 }

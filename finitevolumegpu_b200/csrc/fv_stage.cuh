@@ -1230,8 +1230,8 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
 // soon as the one before has handed out its tasks; instead of the end of that
 // one it waits for the tiles that it reads, as within a launch, so the chain has
 // no gaps: KP07_dimsplit 4096 x 4096 in one launch per 100 steps, in a chain of
-// 18, and in 17 launches that each wait for the end of the one before: 260.8,
-// 261.1 and 265.6 us per step; LxF 84.4, 84.7 and 105.7.  Its CTAs end after the
+// 52, and in 17 launches that each wait for the end of the one before: 260.8,
+// 261.6 and 265.6 us per step; LxF 84.4, 84.8 in 26, and 105.7 in 34.  Its CTAs end after the
 // launch before has ended, so the end of the last launch is that of the run.
 //
 // LOOP: the form for GPUs shared with other simulations of the context.  The

@@ -15,7 +15,7 @@ import finitevolumegpu_b200 as fv
 pytestmark = pytest.mark.gpu
 
 WALLS = {"reflective": 0x03030303, "periodic": 0x02020202, "mixed": 0x02020303}
-CHAIN_CELLS = 1 << 27  # cell updates of one launch (chain_tasks in fv_api.cu)
+CHAIN_CELLS = 1 << 24  # cell updates of one launch beside others (chain_cells in fv_api.cu)
 
 
 def make(ctx, scheme, nx, ny, bc=0x03030303):
@@ -135,14 +135,14 @@ def test_small_simulations_run_side_by_side(ctx):
 
 
 def test_small_simulation_beside_a_large_one(ctx):
-    """20 steps of 256 x 256 wait for a part of the large grid's 100 steps only."""
+    """20 steps of 256 x 256, and one, wait for a part of the large grid's 100 steps only."""
     big, small = make(ctx, "KP07_dimsplit", 4096, 4096), make(ctx, "KP07_dimsplit", 256, 256)
     db, ds = float(big.computeDt()) * 0.3, float(small.computeDt()) * 0.3
     big.simulate(99.5 * db, db)
     t0 = time.perf_counter()
     big.simulate(99.5 * db, db)
     alone = time.perf_counter() - t0
-    stop, waits = threading.Event(), []
+    stop, waits, steps = threading.Event(), [], []
 
     def run_big():
         while not stop.is_set():
@@ -153,11 +153,16 @@ def test_small_simulation_beside_a_large_one(ctx):
         for _ in range(10):
             t0 = time.perf_counter()
             small.simulate(19.5 * ds, ds)
-            waits.append(time.perf_counter() - t0)
+            t1 = time.perf_counter()
+            waits.append(t1 - t0)
+            small.step(np.float32(ds))
+            small.synchronize()
+            steps.append(time.perf_counter() - t1)
         stop.set()
 
     side_by_side([run_big, run_small])
     assert sorted(waits)[5] < 0.3 * alone, (waits, alone)
+    assert sorted(steps)[5] < 0.03 * alone, (steps, alone)
 
 
 def test_steps_on_threads_equal_steps_alone(ctx):
