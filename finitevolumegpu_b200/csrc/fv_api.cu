@@ -625,7 +625,8 @@ struct fv_sim {
     cudaStream_t stream = nullptr;
     alignas(64) StageArgs args;
     size_t smem = 0;         // dynamic shared memory of a launch (stage_smem)
-    LoopForm loop, wide;     // the looping forms (loop_form), once needed
+    LoopForm loop[3];        // the looping forms (loop_form), once needed
+    int n_loop = 0;
     long long launches = 0;  // stage-kernel launches so far
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
@@ -907,27 +908,39 @@ int set_loop_form(fv_sim* s, const KEntry* e, LoopForm* f) {
 //
 // A simulation takes its share of the CTAs that the GPU holds, at most 1.2 times
 // its tiles (stage_smem).  If its share is less, its speed depends on the work
-// that all do, and a tile with short chains gives way to the one of the same
-// scheme with less halo or more cells per thread (28 x 28, unsplit 60 x 28, by
-// 128 threads).  us per step and simulation, 8 threads: EE2D 200 x 600 10.0 with
-// its 12 x 12 tile, 7.0; LxF 512 x 512 4.4 with a CTA per task, 1.5.  Half and
-// twice the share: KP07_dimsplit 1024 x 1024 25.4, 20.0, FORCE 777 x 1333 9.3,
-// 6.9, EE2D 7.2, 9.0.
+// that all do, and a 12 x 12 tile, with short chains but much halo, gives way to
+// 28 x 28 by 224 threads, and this one, if the share is less than a third, to
+// 28 x 28 by 128, with more cells per thread; unsplit, 60 x 28 by 256 or 448
+// threads to 60 x 28 by 128.  us per step and simulation, 4 and 8 threads:
+// KP07_dimsplit 256 x 256 with 12 x 12 only, 28 x 28 by 224 and by 128 3.9 3.0,
+// 4.1 3.1, 4.5 3.7; EE2D 200 x 600 9.9 10.0, 8.7 8.6, 10.3 7.2; LxF 512 x 512 4.4
+// with a CTA per task, 1.5.  With half and twice the share: KP07_dimsplit
+// 1024 x 1024 25.4, 20.0, FORCE 777 x 1333 9.3, 6.9, EE2D 7.2, 9.0.
 int loop_form(fv_sim* s, const LoopForm** form, unsigned* ctas) {
     *form = nullptr;
     const int running = s->ctx->running.load(std::memory_order_relaxed);
     if (running < 2) return FV_OK;
-    if (!s->loop.ke) {
-        FV_TRY(set_loop_form(s, s->ke, &s->loop));
-        const int w = s->ke->split ? 28 : 60;
-        for (const KEntry& e : kTable)
-            if (s->p.variant == 0 && e.scheme == s->scheme && e.W == w && e.H == 28 && e.NT == 128 &&
-                (s->ke->split ? s->ke->W < w : s->ke->W == w && s->ke->NT > 128))
-                FV_TRY(set_loop_form(s, &e, &s->wide));
+    if (s->n_loop == 0) {
+        FV_TRY(set_loop_form(s, s->ke, &s->loop[0]));
+        int n = 1;
+        auto add = [&](int W, int NT) {
+            for (const KEntry& e : kTable)
+                if (s->p.variant == 0 && e.scheme == s->scheme && e.W == W && e.H == 28 && e.NT == NT)
+                    return set_loop_form(s, &e, &s->loop[n++]);
+            return FV_OK;
+        };
+        if (s->ke->split && s->ke->W < 28) FV_TRY(add(28, 224));
+        if (s->ke->split ? s->ke->W < 28 || (s->ke->W == 28 && s->ke->NT > 128) : s->ke->W == 60 && s->ke->NT > 128)
+            FV_TRY(add(s->ke->split ? 28 : 60, 128));
+        s->n_loop = n;
     }
     auto wanted = [](const LoopForm& f) { return (f.grid.x * f.grid.y * 6 + 4) / 5; };
-    const LoopForm* f = &s->loop;
-    if (s->wide.ke && wanted(*f) > f->resident / running) f = &s->wide;
+    const LoopForm* f = &s->loop[0];
+    for (int k = 1; k < s->n_loop; ++k) {
+        const bool latency = s->ke->split && f->ke->W == 28;  // 28 x 28 by 224 threads
+        if (wanted(*f) > (latency ? 3 : 1) * (f->resident / running)) f = &s->loop[k];
+        else break;
+    }
     if (2 * f->grid.x * f->grid.y > 3 * f->resident) return FV_OK;
     *form = f;
     *ctas = std::max(1u, std::min(wanted(*f), f->resident / running));
