@@ -884,6 +884,7 @@ struct StagePlan {
     const float* tail = nullptr;
     int n_tail = 0;
     bool want_cfl = true;
+    bool whole = false;        // one launch, however long
     int row0 = 0, nrows = -1;  // a band of tile rows (one substep)
     const LoopForm* loop = nullptr;  // the looping form, null: a CTA per task
     unsigned loop_ctas = 0;
@@ -993,7 +994,7 @@ int launch_stage(fv_sim* s, const StagePlan& p) {
                                dim3(p.loop->ke->NT), kargs, entry_smem(*p.loop->ke), s->stream));
         ++s->launches;
     } else {
-        const long long most = p.n_sub > 1 ? chain_tasks(s) : tiles;
+        const long long most = p.n_sub > 1 && !p.whole ? chain_tasks(s) : (long long)tiles * p.n_sub;
         // step()'s few substeps: padded where there is nothing else that could run
         // beside them (1024 x 1024 alone 35.7 us instead of 39.0;
         // on 8 threads 22.0 instead of 20.9, 256 x 256 8.2 instead of 6.6)
@@ -1013,8 +1014,8 @@ int launch_stage(fv_sim* s, const StagePlan& p) {
 }
 
 // k steps: the last n_tail of them take the time steps tail[], the others the
-// control block's dt.
-int run_steps(fv_sim* s, long long k, const float* tail, int n_tail, bool want_cfl) {
+// control block's dt.  whole: without chains.
+int run_steps(fv_sim* s, long long k, const float* tail, int n_tail, bool want_cfl, bool whole = false) {
     NvtxRange range("fv steps");
     const long long most = INT_MAX / ((long long)s->grid.x * s->grid.y * s->num_substeps);
     long long full = k - n_tail;
@@ -1024,6 +1025,7 @@ int run_steps(fv_sim* s, long long k, const float* tail, int n_tail, bool want_c
         p.steps = (int)std::min(k, p.loop ? loop_steps(s, *p.loop) : std::max<long long>(1, most));
         p.n_sub = p.steps * s->num_substeps;
         p.explicit_dt = false;
+        p.whole = whole;
         p.full_steps = (int)std::min<long long>(full, p.steps);
         p.tail = tail;
         p.n_tail = p.steps - p.full_steps;
@@ -1372,12 +1374,13 @@ int fv_sim_advance(fv_sim* s, long long n_steps) {
     long long nt = c.nt;
     for (long long left = n_steps; left > 0;) {
         long long k = std::min(left, 100 - nt % 100);
-        // A chain of launches needs a finite dt.
-        if (k * s->num_substeps * s->grid.x * s->grid.y > chain_tasks(s)) {
-            FV_TRY(read_ctl(s));
-            if (!std::isfinite(c.dt)) k = left = 1;  // no step follows it: t is not finite either
-        }
-        FV_TRY(run_steps(s, k, nullptr, 0, (nt + k) % 100 == 0));
+        const long long tasks = (long long)s->num_substeps * s->grid.x * s->grid.y;
+        // A chain of launches needs a dt that is finite.  A later interval's is not
+        // known here: its first step is one launch, which takes any dt, and after a
+        // dt that is not finite no step follows, as t is not finite either.
+        const bool first = k * tasks > chain_tasks(s) && (nt == c.nt ? !std::isfinite(c.dt) : nt % 100 == 0);
+        if (first) k = 1;
+        FV_TRY(run_steps(s, k, nullptr, 0, (nt + k) % 100 == 0, first));
         left -= k;
         nt += k;
     }

@@ -184,3 +184,25 @@ def test_steps_on_threads_equal_steps_alone(ctx):
         assert s.simSteps() == 40 and s.computeDt() == alone.computeDt()
         for x, y in zip(s.download(), want):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("dt", [None, np.inf, np.nan, 0.0, -1.0])
+def test_advance_of_several_intervals_in_chains(ctx, dt):
+    """advance() over three dt intervals on a grid whose runs are chains, against
+    single steps of it; a dt that is not a positive number ends it after the
+    step that it spoils, or before the first."""
+    nx, ny = 1500, 1201
+    a, b = make(ctx, "KP07_dimsplit", nx, ny), make(ctx, "KP07_dimsplit", nx, ny)
+    if dt is None:
+        a.advance(230)
+        while b.simSteps() < 230:
+            b.advance(1)
+        assert a.simSteps() == b.simSteps() == 230 and a.simTime() == b.simTime()
+        for x, y in zip(a.download(), b.download()):
+            assert np.array_equal(x, y)
+        return
+    t, nt, _, cfl = a.get_control()
+    a.set_control(t, 150, np.float32(dt), cfl)  # in the middle of an interval: this dt is used
+    a.advance(200)
+    assert a.simSteps() == (150 if dt <= 0.0 else 151)
+    assert np.isfinite(a.simTime()) == (dt <= 0.0)
