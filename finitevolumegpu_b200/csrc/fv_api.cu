@@ -949,17 +949,15 @@ int loop_form(fv_sim* s, const LoopForm** form, unsigned* ctas) {
 }
 
 // Cell updates of a launch of a chain, which is what other streams wait for at
-// most: 2^24, a tenth of a millisecond, where the context has other simulations
-// or batches, which may run at any time, and 2^26 where it has none.  256 x 256
-// steps beside a 4096 x 4096 run, ms, with a launch per substep, launches of 100
-// steps, and chains of 2^27, 2^26, 2^24 and 2^22: one step 0.15, 13.4, 0.97, 0.52,
-// 0.13, 0.06; two 0.46, 23.8, 1.0, 0.53, 0.15, 0.09; twenty 3.2, 25.5, 2.8, 2.3,
-// 2.1, 2.3.  us per step on 4096 x 4096 in one launch and in the same chains:
-// KP07_dimsplit 260.8, 261.3, 261.6, 261.6, 263.3; LxF 84.4, 84.4, 84.8, 86.9, 95.7.
-int chain_cells(const fv_context* ctx) {
-    return ctx->members.load(std::memory_order_relaxed) > 1 ? 1 << 24 : 1 << 26;
-}
-long long chain_tasks(const fv_sim* s) { return chain_cells(s->ctx) / (s->ke->W * s->ke->H); }
+// most: half a millisecond.  256 x 256 steps beside a 4096 x 4096 run, ms, with a
+// launch per substep, launches of 100 steps, and chains of 2^27, 2^26, 2^25 and
+// 2^24: one step 0.15, 13.4, 0.97, 0.52, 0.26, 0.13; two 0.46, 23.8, 1.0, 0.53,
+// 0.28, 0.15; twenty 3.2, 25.5, 2.8, 2.3, 2.1, 2.1.  What the launches cost, us per
+// step in one and in the same chains: KP07_dimsplit 4096 x 4096 260.8, 261.3,
+// 261.6, 261.4, 261.6; LxF 84.4, 84.4, 84.8, 85.5, 86.9; FORCE 777 x 1333 loses 3 %
+// with 2^24.
+constexpr int kChainCells = 1 << 26;
+long long chain_tasks(const fv_sim* s) { return kChainCells / (s->ke->W * s->ke->H); }
 
 // Steps of a run in the looping form: 2^24 cell updates, after which a run takes
 // the share of the then current number of simulations (a quarter of them loses
@@ -1730,7 +1728,7 @@ int batch_launch(fv_batch* b, int n_steps) {
     }
     const size_t smem = stage_smem(b->ctx, tile, (size_t)b->nwork);
     const long long per_step = (long long)b->nwork * b->num_substeps;
-    const long long chain = chain_cells(b->ctx) / (b->be->W * b->be->H);
+    const long long chain = kChainCells / (b->be->W * b->be->H);
     const int most = (int)std::max<long long>(1, INT_MAX / per_step);  // steps of a run
     for (int left = n_steps; left > 0;) {
         const int steps = std::min(left, most);

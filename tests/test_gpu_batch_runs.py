@@ -39,7 +39,7 @@ def test_long_run_equals_single_steps_and_plain(ctx, scheme):
     a, slots = make(ctx, scheme)
     before = a.launches()
     a.run(STEPS)  # past every end
-    assert a.launches() - before <= 4  # one run of 400 steps, in parts of 2^24 cell updates
+    assert a.launches() - before <= 4  # one run of 400 steps, in parts of 2^26 cell updates
     b, _ = make(ctx, scheme)
     for _ in range(STEPS):
         b.run(1)

@@ -15,7 +15,7 @@ import finitevolumegpu_b200 as fv
 pytestmark = pytest.mark.gpu
 
 WALLS = {"reflective": 0x03030303, "periodic": 0x02020202, "mixed": 0x02020303}
-CHAIN_CELLS = 1 << 24  # cell updates of one launch beside others (chain_cells in fv_api.cu)
+CHAIN_CELLS = 1 << 26  # cell updates of one launch (kChainCells in fv_api.cu)
 
 
 def make(ctx, scheme, nx, ny, bc=0x03030303):
