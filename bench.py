@@ -4,8 +4,9 @@ Workload: KP07_dimsplit shallow water on a 4096 x 4096 FP32 grid, circular dam
 break (h = 1 inside a seeded radius R ~ U(0.1, 0.3) * width, 0.1 outside,
 hu = hv = 0, g = 9.81, reflective walls), stepped with simulate()'s CFL
 schedule (dt recomputed every 100 steps).  One bench step is one full time
-step (two substeps of the whole grid; a launch runs up to 100 steps).  The
-state (2 x 201 MB) is larger than L2, so no flush is needed between steps.
+step (two substeps of the whole grid; a launch is 2^26 cell updates, about two
+steps).  The state (2 x 201 MB) is larger than L2, so no flush is needed between
+steps.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl mine|reference]
 
@@ -319,7 +320,7 @@ def kh_ic(nx, ny, rng, gamma=1.4):
 
 def run_batched(ctx, n_inst=512, seed=4, check=8):
     """Config 4: 512 KP07_dimsplit simulations, sides log-uniform in [64, 1024], bump or dam break,
-    t_end ~ U(5, 50): one batch (one batched launch per run of steps) vs the plain simulators one after another."""
+    t_end ~ U(5, 50): one batch (runs of 16 steps) vs the plain simulators one after another."""
     from finitevolumegpu_b200 import KP07_dimsplit
     from finitevolumegpu_b200.batch import Batch
 

@@ -86,7 +86,8 @@ int scheme_ghost(int scheme) { return (scheme == FV_LXF || scheme == FV_FORCE ||
 // The kernels of a table row, in the part that compiles them.
 template <int S, int W, int H, int NT, int VAR = 0, int LPT = 1>
 constexpr StageFns stage_fn() {
-    if constexpr (S == kPart) return {fv::stage_kernel<S, W, H, NT, VAR, LPT>, fv::stage_kernel<S, W, H, NT, VAR, LPT, true>};
+    if constexpr (S == kPart)
+        return {fv::stage_kernel<S, W, H, NT, VAR, LPT>, fv::stage_kernel<S, W, H, NT, VAR, LPT, true>};
     else return {};
 }
 template <int S, int... P>
@@ -996,7 +997,8 @@ int launch_stage(fv_sim* s, const StagePlan& p) {
         // step()'s few substeps: padded where there is nothing else that could run
         // beside them (1024 x 1024 alone 35.7 us instead of 39.0;
         // on 8 threads 22.0 instead of 20.9, 256 x 256 8.2 instead of 6.6)
-        const bool padded = p.n_sub > s->num_substeps || (p.n_sub > 1 && s->ctx->members.load(std::memory_order_relaxed) == 1);
+        const bool padded = p.n_sub > s->num_substeps ||
+                            (p.n_sub > 1 && s->ctx->members.load(std::memory_order_relaxed) == 1);
         for (long long left = (long long)tiles * p.n_sub; left > 0;) {
             const unsigned ctas = (unsigned)std::min(left, most);
             left -= ctas;

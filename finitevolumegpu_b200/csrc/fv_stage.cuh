@@ -1231,18 +1231,19 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
 // one it waits for the tiles that it reads, as within a launch, so the chain has
 // no gaps: KP07_dimsplit 4096 x 4096 in one launch per 100 steps, in a chain of
 // 52, and in 17 launches that each wait for the end of the one before: 260.8,
-// 261.6 and 265.6 us per step; LxF 84.4, 84.8 in 26, and 105.7 in 34.  Its CTAs end after the
-// launch before has ended, so the end of the last launch is that of the run.
+// 261.6 and 265.6 us per step; LxF 84.4, 84.8 in 26, and 105.7 in 34.  Its CTAs
+// end after the launch before has ended, so the end of the last launch is that of
+// the run.
 //
 // LOOP: the form for GPUs shared with other simulations of the context.  The
 // launch has fewer CTAs than tasks (loop_form) and each takes task after task,
 // so that none is queued behind others and simulations run beside each other.
 // us per step and simulation with 1, 2, 4 and 8 threads that each run one:
 //                             a launch per substep    CTA per task            LOOP from 2 on
-//   KP07_dimsplit 64 x 48     14.7  7.8  4.0  2.1     7.7  7.3  7.3  7.2      7.7  4.4  2.0  1.2
-//   KP07_dimsplit 256 x 256   16.1  8.4  4.7  3.3     10.2 9.7  9.8  9.7      10.0 6.1  3.8  3.0
-//   FORCE 777 x 1333          14.4  9.3  6.0  6.3     8.1  7.7  7.7  7.6      8.1  6.9  6.7  6.9
-//   KP07_dimsplit 1024 x 1024 35.6 26.8 19.8 19.7     21.8 21.4 21.3 21.3     21.7 21.3 19.8 20.1
+//   KP07_dimsplit 64 x 48     14.7  7.8  4.0  2.1     7.7  7.3  7.3  7.2      7.7  4.4  2.0  1.1
+//   KP07_dimsplit 256 x 256   16.1  8.4  4.7  3.3     10.2 9.7  9.8  9.7      8.7  5.7  4.0  3.1
+//   FORCE 777 x 1333          14.4  9.3  6.0  6.3     8.1  7.7  7.7  7.6      8.1  6.7  6.6  6.9
+//   KP07_dimsplit 1024 x 1024 35.6 26.8 19.8 19.7     21.8 21.4 21.3 21.3     21.6 21.9 20.3 20.3
 // A CTA keeps nothing but its task between two of them (per_task, clear): with
 // what the compiler would keep, KP07_dimsplit's 28 x 28 tile takes 128 registers
 // instead of 71.
@@ -1259,7 +1260,7 @@ __host__ __device__ constexpr int compiled_blocks(int scheme, int W, int H, int 
 //   HLL2           16.9  12.3   9.1    41.4  27.5  27.5    115  89.4  85.6    376   349   334
 //   WAF            18.7  14.7  10.4    52.2  37.4  37.7    157   132   128    545   514   504
 //   KP07           18.7  15.4  10.7    36.6  21.9  19.8    103  81.3  74.6    348   324   301
-//   KP07_dimsplit  15.1  10.5   9.9    34.5  22.0  21.7   84.7  67.3  66.5    282   264   261
+//   KP07_dimsplit  15.1  10.5   8.2    34.5  22.0  21.5   84.7  67.3  66.7    282   264   261
 //   EE2D           18.4  13.5  10.0    46.5  31.1  29.6    128   109   104    440   422   403
 // (FORCE before and now: 6.5 3.4, 13.3 8.0, 35.3 26.6, 111 105).
 template <int SCHEME, int W, int H, int NT, int VAR = 0, int LPT = 1, bool LOOP = false>
